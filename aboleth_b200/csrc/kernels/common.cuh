@@ -27,37 +27,6 @@ __device__ __forceinline__ void set_status(unsigned long long *status,
         status[1] = detail;
 }
 
-// ---- launches that overlap the end of the kernel before them --------------------------
-//
-// A layer is a chain of short kernels; between two of them the device otherwise drains, takes the next launch and
-// runs its prologue (1 to 3 us).  A kernel launched by `launch_chained` may start while the one before it in the
-// stream finishes, so it calls `grid_wait` before it touches any global memory: that returns when every kernel
-// before it has completed and its writes are visible.  `grid_next` lets the kernel after it start early in turn; a
-// kernel that never calls it, or is launched the ordinary way, is simply not overlapped.
-//
-// Back-to-back passes: quantise, pack and multiply 1000 x 8192 x 3584 block-scaled 40.7 -> 37.1 us, 32 x 3584 x 8192
-// 17.7 -> 16.6, the bf16 one-rank layer of 2999 tokens 50.9 -> 46.6, the 4096-token layer 225 -> 222.  The grouped
-// GEMMs of few-row experts are launched the ordinary way: chained as well, the e4m3 MoE layer of 24 tokens took 304
-// us against 296 (299 without any chaining).
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <typename... Params, typename... Args>
-inline void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, std::size_t smem, cudaStream_t stream,
-                           Args &&...args) {
-    cudaLaunchConfig_t config{};
-    config.gridDim = grid;
-    config.blockDim = block;
-    config.dynamicSmemBytes = smem;
-    config.stream = stream;
-    cudaLaunchAttribute attribute{};
-    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute.val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = &attribute;
-    config.numAttrs = 1;
-    cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
-}
-
 inline int launch_result(const char *what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

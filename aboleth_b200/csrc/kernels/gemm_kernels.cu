@@ -190,8 +190,7 @@ int launch_grouped(const void *a, const void *w, void *c, const int *counts, con
     const long long column_bytes = static_cast<long long>(BN) * k * 2;
     const int group_n = static_cast<int>(std::max(1LL, std::min<long long>(tiles_n, (48LL << 20) / column_bytes)));
     Policy p{static_cast<__nv_bfloat16 *>(c), counts, offsets, experts, n, k, n, tiles_n, group_n, 0, 0};
-    // The tile count depends on counts the host never reads: a persistent grid that fills the device.  Not chained
-    // (see launch_chained).
+    // The tile count depends on counts the host never reads: a persistent grid that fills the device.
     if constexpr (CTAS == 2) {
         using G = pair::PairGeometry<BN>;
         auto kernel = gemm_pair_kernel<OpBf16, BN, Policy>;
@@ -348,8 +347,6 @@ __device__ __forceinline__ unsigned ue8m0_of(float scale, unsigned long long *st
 // bytes: byte (r % 32) * 16 + (r / 32) * 4 + s for row r of the block, the same value for s = 0..3.
 __global__ void pack_scales_a_kernel(const float *scales, long long ld, std::uint32_t *out, int rows,
                                      int k_blocks, unsigned long long *status) {
-    ab::grid_next();
-    ab::grid_wait();
     const long long row_blocks = mx::mx_row_blocks(rows);
     const long long total = row_blocks * k_blocks * 128;
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -368,8 +365,6 @@ __global__ void pack_scales_a_kernel(const float *scales, long long ld, std::uin
 // (256- and 192-column tiles both) finds its two atoms at g and g + 2.  `granules` per K block.
 __global__ void pack_scales_b_kernel(const float *scales, long long ld, std::uint32_t *out, int n_blocks,
                                      int granules, int k_blocks, unsigned long long *status) {
-    ab::grid_next();
-    ab::grid_wait();
     const long long total = static_cast<long long>(k_blocks) * granules * 128;
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -426,14 +421,13 @@ int launch_split(const DenseArgs &d, int split, cudaStream_t stream) {
     config.blockDim = dim3(kThreads);
     config.dynamicSmemBytes = G::kSmemBytes;
     config.stream = stream;
-    cudaLaunchAttribute attributes[2] = {};
-    attributes[0].id = cudaLaunchAttributeClusterDimension;
-    attributes[0].val.clusterDim.x = p.split;
-    attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
-    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch_chained
-    attributes[1].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attributes;
-    config.numAttrs = 2;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = p.split;
+    attribute.val.clusterDim.y = 1;
+    attribute.val.clusterDim.z = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&config, kernel, map_x, map_y, p);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -510,7 +504,7 @@ int launch_pair(const DenseArgs &d, cudaStream_t stream) {
     const int group_n = static_cast<int>(std::max(1LL, std::min<long long>(tiles_n, (48LL << 20) / column_bytes)));
     const PlainPolicy<NT> p{static_cast<__nv_bfloat16 *>(d.c), d.m, d.n, d.k, d.ldc, tiles_n, tiles, group_n, Op::kBK,
                         d.alpha};
-    ab::launch_chained(kernel, 2 * std::min(tiles, resident), kThreads, G::kSmemBytes, stream, map_a, map_b, p, d.status);
+    kernel<<<2 * std::min(tiles, resident), kThreads, G::kSmemBytes, stream>>>(map_a, map_b, p, d.status);
     return ab::launch_result(Op::kBK == 64 ? "gemm_bf16 (CTA pairs)" : "gemm_e4m3 (CTA pairs)");
 }
 
@@ -720,7 +714,7 @@ int launch_mx_pair(const void *a, const void *sfa, const void *b, const void *sf
     if (resident < 1)
         return -3;
     const int pairs = static_cast<int>(std::min<long long>(tiles, resident));
-    ab::launch_chained(kernel, 2 * pairs, kThreads, G::kSmemBytes, stream, map_a, map_b, map_sfa, map_sfb, policy, k_blocks, granules,
+    kernel<<<2 * pairs, kThreads, G::kSmemBytes, stream>>>(map_a, map_b, map_sfa, map_sfb, policy, k_blocks, granules,
                                                            status);
     return ab::launch_result("gemm_e4m3_mx (CTA pairs)");
 }
@@ -814,10 +808,10 @@ AB_EXPORT int ab_mx_pack_scales(const float *scales, long long ld, void *out, in
         return -1;
     const int k_blocks = k / 128;
     if (which == 0) {
-        ab::launch_chained(pack_scales_a_kernel, 148, 256, 0, stream, scales, ld, static_cast<std::uint32_t *>(out), rows,
+        pack_scales_a_kernel<<<148, 256, 0, stream>>>(scales, ld, static_cast<std::uint32_t *>(out), rows,
                                                       k_blocks, status);
     } else {
-        ab::launch_chained(pack_scales_b_kernel, 148, 256, 0, stream, scales, ld, static_cast<std::uint32_t *>(out),
+        pack_scales_b_kernel<<<148, 256, 0, stream>>>(scales, ld, static_cast<std::uint32_t *>(out),
                                                       (rows + 127) / 128, mx_granules(rows), k_blocks, status);
     }
     return ab::launch_result("mx_pack_scales");
@@ -847,7 +841,7 @@ int launch_mx(const DenseArgs &d, cudaStream_t stream) {
             return -3;
         const mx::ScaleFactors sf{static_cast<const std::uint8_t *>(d.sfa), static_cast<const std::uint8_t *>(d.sfb),
                                   d.k / 128, mx_granules(d.n)};
-        ab::launch_chained(kernel, std::min(p.tiles_total, sm_count()), kThreads, G::kSmemBytes, stream, map_a, map_b, p, sf, d.status);
+        kernel<<<std::min(p.tiles_total, sm_count()), kThreads, G::kSmemBytes, stream>>>(map_a, map_b, p, sf, d.status);
         return ab::launch_result("gemm_e4m3_mx");
     }
 }

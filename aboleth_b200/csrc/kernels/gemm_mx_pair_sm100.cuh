@@ -103,8 +103,6 @@ __device__ __forceinline__ void gemm_mx_mainloop_pair(Policy &policy, const Maps
     cluster_sync();  // both CTAs' barriers exist before anything is signalled across
     tc_fence_after();
     const std::uint32_t tmem_base = st.tmem_base;
-    ab::grid_next();
-    ab::grid_wait();
 
     if (warp == 0) {
         // ---------------- producer (both CTAs): operand tiles and scale-factor atoms ----------------

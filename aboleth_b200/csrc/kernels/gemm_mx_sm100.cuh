@@ -210,8 +210,6 @@ __device__ __forceinline__ void gemm_mx_mainloop(Policy &policy, const CUtensorM
     __syncthreads();
     tc_fence_after();
     const std::uint32_t tmem_base = st.tmem_base;
-    ab::grid_next();
-    ab::grid_wait();
 
     if (warp == 0) {
         // ---------------- producer: TMA tiles and scale-factor atoms ----------------

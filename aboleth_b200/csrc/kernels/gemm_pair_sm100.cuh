@@ -225,8 +225,6 @@ __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtenso
     cluster_sync();  // both CTAs' barriers exist before anything is signalled across
     tc_fence_after();
     const std::uint32_t tmem_base = st.tmem_base;
-    ab::grid_next();
-    ab::grid_wait();
 
     // Accumulator slot (TMEM half) and barrier parity of tile `it`.
     auto slot_of = [](int it) { return it & 1; };

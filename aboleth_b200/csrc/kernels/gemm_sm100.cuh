@@ -387,8 +387,6 @@ __device__ __forceinline__ void gemm_mainloop(Policy &policy, const CUtensorMap 
     __syncthreads();
     tc_fence_after();
     const std::uint32_t tmem_base = st.tmem_base;
-    ab::grid_next();
-    ab::grid_wait();
 
     // Accumulator slot (TMEM half) and barrier parity of half `h` of tile `it`.
     auto slot_of = [](int it, int h) { return HALVES == 1 ? (it & 1) : h; };

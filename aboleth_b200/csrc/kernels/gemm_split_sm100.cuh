@@ -142,8 +142,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const std::uint32_t tmem = st.tmem_base;
-    ab::grid_next();
-    ab::grid_wait();
 
     // Whole-warp loops, one elected lane around the instructions (see elect_one).
     if (warp == 0) {

@@ -390,8 +390,6 @@ __device__ __forceinline__ void finish_dispatch(const DispatchParams &p, std::ui
 // BY_WARP: one warp per token (throughput, token-ordered slots) or one CTA per token (latency).
 template <bool BY_WARP>
 __global__ void __launch_bounds__(kThreads, 4) ep_dispatch_kernel(const __grid_constant__ DispatchParams p) {
-    ab::grid_next();
-    ab::grid_wait();
     const EpGeometry &g = p.g;
     __shared__ int s_id[kMaxTopK];
     __shared__ float s_w[kMaxTopK];
@@ -730,8 +728,6 @@ __device__ __forceinline__ void publish_local(const DispatchParams &p, std::uint
 
 template <bool FP8>
 __global__ void __launch_bounds__(kThreads, 5) ep_dispatch_local_kernel(const __grid_constant__ DispatchParams p) {
-    ab::grid_next();
-    ab::grid_wait();
     const EpGeometry &g = p.g;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int words = meta_words(g);
@@ -1031,8 +1027,6 @@ __device__ __forceinline__ bool reduce_token_by_warp(const CombineParams &p, int
 }
 
 __global__ void __launch_bounds__(kThreads, 3) ep_combine_kernel(const __grid_constant__ CombineParams p) {
-    ab::grid_next();
-    ab::grid_wait();
     const EpGeometry &g = p.g;
     __shared__ int s_flag;
     __shared__ int s_rows[kMaxTopK];
@@ -1270,8 +1264,6 @@ __global__ void __launch_bounds__(kThreads, 3) ep_combine_kernel(const __grid_co
 // places, of the general kernel (whose second pass adds a lone partial to zero).
 template <bool WEIGHTED, int kPieces>
 __global__ void __launch_bounds__(kThreads, kPieces == 4 ? 4 : 3) ep_combine_local_kernel(const __grid_constant__ CombineParams p, int parts) {
-    ab::grid_next();
-    ab::grid_wait();
     const EpGeometry &g = p.g;
     const int lane = threadIdx.x & 31;
     const int vecs = g.hidden / 8, groups = (vecs + 31) / 32;
@@ -1346,8 +1338,6 @@ __global__ void __launch_bounds__(kThreads, kPieces == 4 ? 4 : 3) ep_combine_loc
 __global__ void __launch_bounds__(kThreads) quant_fp8_kernel(
     const std::uint32_t *x, std::uint8_t *q, float *scales, int rows, int hidden, int group,
     float amax_floor, int round_scale) {
-    ab::grid_next();
-    ab::grid_wait();
     const int chunks = hidden / 16;
     const int lanes_per_group = group / 16;
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -1377,8 +1367,6 @@ template <typename Logit>
 __global__ void __launch_bounds__(kThreads) router_topk_kernel(
     const Logit *logits, int *ids, float *weights, int tokens, int experts, int top_k,
     int renormalize) {
-    ab::grid_next();
-    ab::grid_wait();
     const int warp = (blockIdx.x * kThreads + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp >= tokens)
@@ -1398,8 +1386,6 @@ __global__ void __launch_bounds__(kThreads) router_topk_kernel(
 // group the rows of source s follow those of the sources before it.  One CTA; experts <= 1024.
 __global__ void __launch_bounds__(1024) expert_offsets_kernel(
     const int *counts, int *offsets, int *total, int sources, int experts, int align) {
-    ab::grid_next();
-    ab::grid_wait();
     // Warp scans and one scan of the 32 warp totals: two barriers (a scan over shared memory took twenty).
     __shared__ int s_warp[32];
     const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
@@ -1448,8 +1434,6 @@ __global__ void __launch_bounds__(kThreads) permute_kernel(
     const unsigned long long *recv_counts, int *perm_row, int world, int capacity, int top_k,
     int row_bytes, int cols, int src_scale_stride, int offset_stride, std::uint32_t *dst_packed,
     unsigned long long *status) {
-    ab::grid_next();
-    ab::grid_wait();
     const int total = world * capacity;
     for (int row = blockIdx.x; row < total; row += gridDim.x) {
         const int srcr = row / capacity;
@@ -1487,8 +1471,6 @@ __global__ void __launch_bounds__(kThreads) unpermute_kernel(
     const std::uint32_t *y, std::uint32_t *out, const int *expert_ids, const int *expert_pos,
     const float *expert_weights, const int *offsets, const unsigned long long *recv_counts,
     int world, int capacity, int top_k, int hidden, int offset_stride) {
-    ab::grid_next();
-    ab::grid_wait();
     const int total = world * capacity;
     const int vecs = hidden / 8;
     for (int row = blockIdx.x; row < total; row += gridDim.x) {
@@ -1532,8 +1514,6 @@ __global__ void __launch_bounds__(kThreads) standin_expert_kernel(
     const int *expert_ids, const float *expert_weights, const int *expert_pos, const int *offsets,
     const unsigned long long *recv_counts, int world, int capacity, int top_k, int hidden, int group,
     int value_fp8, int offset_stride) {
-    ab::grid_next();
-    ab::grid_wait();
     const int total = world * capacity;
     __shared__ float s_coef[kMaxTopK];
     __shared__ int s_out[kMaxTopK];
@@ -1716,16 +1696,16 @@ AB_EXPORT int ab_ep_dispatch(const int *ints, float amax_floor, const std::uint6
         grid = std::max(1, std::min(requested > 0 ? requested : p.num_tokens, held));
         g_last_grid[0] = grid;
         if (p.g.value_fp8)
-            ab::launch_chained(ep_dispatch_local_kernel<true>, grid, kThreads, 0, stream, p);
+            ep_dispatch_local_kernel<true><<<grid, kThreads, 0, stream>>>(p);
         else
-            ab::launch_chained(ep_dispatch_local_kernel<false>, grid, kThreads, 0, stream, p);
+            ep_dispatch_local_kernel<false><<<grid, kThreads, 0, stream>>>(p);
         return ab::launch_result("ep_dispatch");
     }
     g_last_grid[0] = grid;
     if (p.by_warp)
-        ab::launch_chained(ep_dispatch_kernel<true>, grid, kThreads, 0, stream, p);
+        ep_dispatch_kernel<true><<<grid, kThreads, 0, stream>>>(p);
     else
-        ab::launch_chained(ep_dispatch_kernel<false>, grid, kThreads, 0, stream, p);
+        ep_dispatch_kernel<false><<<grid, kThreads, 0, stream>>>(p);
     return ab::launch_result("ep_dispatch");
 }
 
@@ -1782,11 +1762,11 @@ AB_EXPORT int ab_ep_combine(const int *ints, float amax_floor, const std::uint64
         g_last_grid[1] = static_cast<int>(std::max(1LL, (items + kWarps - 1) / kWarps));
         const auto kernel = !p.weighted ? ep_combine_local_kernel<false, 8>
                             : parts * 2 > groups ? ep_combine_local_kernel<true, 1> : ep_combine_local_kernel<true, 4>;
-        ab::launch_chained(kernel, g_last_grid[1], kThreads, 0, stream, p, parts);
+        kernel<<<g_last_grid[1], kThreads, 0, stream>>>(p, parts);
         return ab::launch_result("ep_combine");
     }
     g_last_grid[1] = resident_grid<ep_combine_kernel>(grid);
-    ab::launch_chained(ep_combine_kernel, g_last_grid[1], kThreads, 0, stream, p);
+    ep_combine_kernel<<<g_last_grid[1], kThreads, 0, stream>>>(p);
     return ab::launch_result("ep_combine");
 }
 
@@ -1795,7 +1775,7 @@ AB_EXPORT int ab_quant_fp8(const void *x, void *q, float *scales, int rows, int 
     if (rows < 1 || hidden % 16 || group % 16 || hidden % group || (group & (group - 1)) || group > 512)
         return -1;
     const int grid = rows < 148 * 8 ? rows : 148 * 8;
-    ab::launch_chained(quant_fp8_kernel, grid, kThreads, 0, stream, static_cast<const std::uint32_t *>(x),
+    quant_fp8_kernel<<<grid, kThreads, 0, stream>>>(static_cast<const std::uint32_t *>(x),
                                                     static_cast<std::uint8_t *>(q), scales, rows,
                                                     hidden, group, amax_floor, round_scale);
     return ab::launch_result("quant_fp8");
@@ -1808,7 +1788,7 @@ static int launch_router_topk(const Logit *logits, int *ids, float *weights, int
         top_k > kMaxTopK || top_k > experts)
         return -1;
     const int grid = (tokens * 32 + kThreads - 1) / kThreads;
-    ab::launch_chained(router_topk_kernel<Logit>, grid, kThreads, 0, stream, logits, ids, weights, tokens, experts, top_k, renormalize);
+    router_topk_kernel<<<grid, kThreads, 0, stream>>>(logits, ids, weights, tokens, experts, top_k, renormalize);
     return ab::launch_result("router_topk");
 }
 
@@ -1828,7 +1808,7 @@ AB_EXPORT int ab_expert_offsets(const int *counts, int *offsets, int *total, int
                                 int align, cudaStream_t stream) {
     if (experts < 1 || experts > 1024 || sources < 1)
         return -1;
-    ab::launch_chained(expert_offsets_kernel, 1, (experts + 31) / 32 * 32, 0, stream, counts, offsets, total, sources, experts, align);
+    expert_offsets_kernel<<<1, (experts + 31) / 32 * 32, 0, stream>>>(counts, offsets, total, sources, experts, align);
     return ab::launch_result("expert_offsets");
 }
 
@@ -1840,7 +1820,7 @@ static int launch_permute(const void *src, void *dst, const float *src_scales, f
         return -1;
     const int total = world * capacity;
     const int grid = total < 148 * 8 ? total : 148 * 8;
-    ab::launch_chained(permute_kernel, grid, kThreads, 0, stream, 
+    permute_kernel<<<grid, kThreads, 0, stream>>>(
         static_cast<const std::uint8_t *>(src), static_cast<std::uint8_t *>(dst), src_scales, dst_scales, expert_ids,
         expert_pos, offsets, recv_counts, perm_row, world, capacity, top_k, row_bytes, cols,
         src_scale_stride > 0 ? src_scale_stride : cols, offset_stride, static_cast<std::uint32_t *>(dst_packed), status);
@@ -1876,7 +1856,7 @@ AB_EXPORT int ab_unpermute(const void *y, void *out, const int *expert_ids, cons
         return -1;
     const int total = world * capacity;
     const int grid = total < 148 * 8 ? total : 148 * 8;
-    ab::launch_chained(unpermute_kernel, grid, kThreads, 0, stream, 
+    unpermute_kernel<<<grid, kThreads, 0, stream>>>(
         static_cast<const std::uint32_t *>(y), static_cast<std::uint32_t *>(out), expert_ids,
         expert_pos, expert_weights, offsets, recv_counts, world, capacity, top_k, hidden, offset_stride);
     return ab::launch_result("unpermute");
@@ -1892,7 +1872,7 @@ AB_EXPORT int ab_standin_expert(const void *payload, const float *scales, int sc
         return -1;
     const int total = world * capacity;
     const int grid = total < 148 * 8 ? total : 148 * 8;
-    ab::launch_chained(standin_expert_kernel, grid, kThreads, 0, stream, 
+    standin_expert_kernel<<<grid, kThreads, 0, stream>>>(
         static_cast<const std::uint8_t *>(payload), scales,
         scale_stride > 0 ? scale_stride : hidden / group, static_cast<std::uint32_t *>(y),
         expert_ids, expert_weights, expert_pos, offsets, recv_counts, world, capacity, top_k, hidden,

@@ -394,9 +394,9 @@ def test_pair_tiles_of_both_widths_are_exact_on_integers(m, n, k):
 
 
 def test_chained_launches_see_what_the_kernels_before_them_wrote():
-    """Quantise, pack and multiply in a row, each kernel allowed to start before the one before it has ended, over
-    buffers that the next round overwrites: the results are those of the same calls with a synchronisation after each,
-    also when the chain is captured in a graph and when another stream runs one at the same time."""
+    """Quantise, pack and multiply in a row, with nothing waiting in between, over buffers that the next round overwrites:
+    the results are those of the same calls with a synchronisation after each, also when the chain is captured in a graph
+    and when another stream runs one at the same time."""
     from aboleth_b200.ops import gemm_bf16, gemm_e4m3_mx, pack_scales_mx, quant_fp8
 
     m, n, k = 257, 640, 512
@@ -441,3 +441,34 @@ def test_chained_launches_see_what_the_kernels_before_them_wrote():
     torch.cuda.synchronize()
     for result in (got, other, again, graphed):
         assert torch.equal(result, want)
+
+
+@pytest.mark.parametrize("m,n", [(1000, 8192), (905, 8136)])
+def test_block_scaled_pair_loop_back_to_back(m, n):
+    """Quantise, pack and multiply on two input sets in turn, with no wait in between, at sizes whose product takes the
+    CTA-pair loop with two tiles for most pairs (4 x 32 tiles on 74 pairs), ragged in both directions the second time.
+    The activations are small integers and the weights' scales powers of two: the product is exact, so the outputs are
+    the fp32 product rounded once."""
+    from aboleth_b200.ops import check_gemm_status, gemm_e4m3_block_scaled, pack_scales_mx, quant_fp8
+
+    k, fp8 = 1024, torch.float8_e4m3fn
+    g = torch.Generator(device="cuda").manual_seed(m)
+    b_s = torch.exp2(torch.randint(-2, 3, (-(-n // 128), k // 128), generator=g, device="cuda").float())
+    b = torch.randint(-2, 3, (n, k), generator=g, device="cuda").float()
+    packed = pack_scales_mx(b_s, n, k, weight=True)
+    full = b * b_s.repeat_interleave(128, dim=0)[:n].repeat_interleave(128, dim=1)
+    sets, want = [], []
+    for _ in range(2):
+        x = torch.randint(-7, 8, (m, k), generator=g, device="cuda").float()
+        sets.append(x.to(torch.bfloat16))
+        want.append((x @ full.t()).to(torch.bfloat16))
+    b, got = b.to(fp8), []
+    for i in range(40):
+        q, scales = quant_fp8(sets[i % 2], round_scale=True)
+        out = gemm_e4m3_block_scaled(q, scales, b, b_s, b_packed=packed)
+        if i >= 36:
+            got.append(out)
+    torch.cuda.synchronize()
+    check_gemm_status("cuda")
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 2])
