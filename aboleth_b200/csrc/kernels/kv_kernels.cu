@@ -215,9 +215,10 @@ __global__ void __launch_bounds__(512, 2) kv_push_pages_kernel(const __grid_cons
 // One transfer: page i of `src` (of the producer's pool: `layers` layers, `pool_layer` bytes apart) goes to page
 // dst[i] of the consumer's slot (`slots`: its layer 0, layers `slot_layer` bytes apart); group g of `per_group`
 // layers is published in the cell at cells + g * cell_stride.  `src` and `dst` are host arrays, read before the
-// call returns.  arrivals: device u32 [groups], zeroed.  A run (consecutive pages on both sides) starts inside the
-// pool; a negative page counts from its end.  runs: how many were found; -3 when they are more than one launch
-// carries (256), -4 when a run starts outside the pool; nothing was launched then.
+// call returns.  arrivals: device u32 [groups], zeroed.  Every page of `src` lies inside the pool, where a negative one
+// counts from its end, and every page of `dst` inside the slot.  A run is consecutive pages on both sides, so none
+// continues from the pool's last page to page 0.  runs: how many were found; -3 when they are more than one launch
+// carries (256), -4 when a page of `src`, -5 when a page of `dst` is outside; nothing was launched then.
 AB_EXPORT int ab_kv_push_pages(const long long *src, const long long *dst, int pages, const void *pool, int layers,
                                int blocks, std::uint64_t pool_layer, std::uint64_t page_bytes, std::uint64_t slots,
                                std::uint64_t slot_layer, std::uint64_t cells, std::uint64_t cell_stride, int per_group,
@@ -229,14 +230,20 @@ AB_EXPORT int ab_kv_push_pages(const long long *src, const long long *dst, int p
         return -1;
     KvPages p;
     int n = 0;
+    const long long slot_pages = static_cast<long long>(slot_layer / page_bytes);
+    long long last_from = -1;
     for (int i = 0; i < pages; ++i) {
-        if (i > 0 && src[i] == src[i - 1] + 1 && dst[i] == dst[i - 1] + 1)
-            continue;
-        if (n == kMaxRuns)
-            return -3;
         const long long from = src[i] < 0 ? src[i] + blocks : src[i];
         if (from < 0 || from >= blocks)
             return -4;
+        if (dst[i] < 0 || dst[i] >= slot_pages)
+            return -5;
+        const bool extends = i > 0 && from == last_from + 1 && dst[i] == dst[i - 1] + 1;
+        last_from = from;
+        if (extends)
+            continue;
+        if (n == kMaxRuns)
+            return -3;
         p.run[n++] = KvRun{static_cast<int>(from), static_cast<int>(dst[i]), i};
     }
     *runs = n;
@@ -249,8 +256,7 @@ AB_EXPORT int ab_kv_push_pages(const long long *src, const long long *dst, int p
     p.misaligned = -1;
     if (((reinterpret_cast<std::uint64_t>(pool) | slots | pool_layer | slot_layer | page_bytes) & 15) != 0)
         for (int i = 0; i < layers * n && p.misaligned < 0; ++i) {
-            const std::uint64_t layer = i / n, from = p.run[i % n].src;
-            const std::uint64_t to = static_cast<std::uint64_t>(static_cast<long long>(p.run[i % n].dst));
+            const std::uint64_t layer = i / n, from = p.run[i % n].src, to = p.run[i % n].dst;
             const std::uint64_t a = reinterpret_cast<std::uint64_t>(pool) + layer * pool_layer + from * page_bytes;
             if (((a | (slots + layer * slot_layer + to * page_bytes)) & 15) != 0)
                 p.misaligned = i;

@@ -19,12 +19,15 @@ declare("ab_memcpy_async", [_VP, _VP, _U64, _VP])
 
 def canonicalize_block_runs(src_blocks: Sequence[int], dst_blocks: Sequence[int]) -> list[tuple[int, int, int]]:
     """Merge (src, dst) block pairs into maximal runs ``(src_start, dst_start, length)`` where
-    both sides are consecutive (reference: python/aboleth/kv/copy.py ``canonicalize_block_runs``)."""
+    both sides are consecutive (reference: python/aboleth/kv/copy.py ``canonicalize_block_runs``).  A negative
+    block, one counted from the end, is never followed by block 0 in a run: the next block after the last
+    one is not the first."""
     if len(src_blocks) != len(dst_blocks):
         raise ValueError("source and destination block lists differ in length")
     runs: list[tuple[int, int, int]] = []
     for s, d in zip(src_blocks, dst_blocks):
-        if runs and runs[-1][0] + runs[-1][2] == s and runs[-1][1] + runs[-1][2] == d:
+        if runs and runs[-1][0] + runs[-1][2] == s and runs[-1][1] + runs[-1][2] == d and not (
+                (s == 0 and runs[-1][0] < 0) or (d == 0 and runs[-1][1] < 0)):
             runs[-1] = (runs[-1][0], runs[-1][1], runs[-1][2] + 1)
         else:
             runs.append((int(s), int(d), 1))
@@ -67,7 +70,8 @@ def push_pages(src_blocks: Sequence[int], dst_pages: Sequence[int], *, pool: tor
                workers: int, threads: int) -> int | None:
     """Launch the push of one transfer, every layer of ``pool`` (``[layers, blocks, page_bytes]``): the runs are found
     and the launch is made in one native call.  Returns the number of runs, or None (nothing launched) when there are
-    more than one launch carries."""
+    more than one launch carries.  A page outside the pool is an ``IndexError``, one outside the slot a
+    ``ValueError``."""
     n = len(src_blocks)
     if len(dst_pages) != n:
         raise ValueError("source and destination block lists differ in length")
@@ -76,12 +80,14 @@ def push_pages(src_blocks: Sequence[int], dst_pages: Sequence[int], *, pool: tor
     layers, blocks, page_bytes = pool.shape
     src, dst = array(*map(int, src_blocks)), array(*map(int, dst_pages))
     rc = call_rc("ab_kv_push_pages", src, dst, n, ptr(pool), layers, blocks, pool.stride(0), page_bytes, slots,
-                          slot_layer, cells, cell_stride, per_group, epoch, ptr(arrivals), ptr(status), workers, threads,
-                          ctypes.byref(runs), stream_ptr())
+                 slot_layer, cells, cell_stride, per_group, epoch, ptr(arrivals), ptr(status), workers, threads,
+                 ctypes.byref(runs), stream_ptr())
     if rc == -3:
         return None
     if rc == -4:
         raise IndexError(f"a source block is outside the pool of {blocks}")
+    if rc == -5:
+        raise ValueError("the transfer does not fit the consumer's slot")
     if rc != 0:
         raise RuntimeError(f"ab_kv_push_pages failed with code {rc} (bad arguments or CUDA launch error)")
     return runs.value

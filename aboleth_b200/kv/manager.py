@@ -71,7 +71,7 @@ class CompiledKVTransferManager:
         (run, layer) batches launched.  ``epoch`` is the readiness value the consumer waits for."""
         l, rank = self.layout, self.world.rank
         dst_pages = list(range(len(src_blocks))) if dst_pages is None else list(dst_pages)
-        if max(dst_pages, default=0) >= l.slot_pages:
+        if max(dst_pages, default=0) >= l.slot_pages or min(dst_pages, default=0) < 0:
             raise ValueError("the transfer does not fit the consumer's slot")
         if len(src_blocks) == 0:
             raise ValueError("a transfer needs at least one block")
@@ -88,7 +88,9 @@ class CompiledKVTransferManager:
             if found is not None:
                 return found * l.layers
         # More runs than one launch's arguments hold: one batch per (run, layer), uploaded.
-        runs = kvcopy.canonicalize_block_runs(src_blocks, dst_pages)
+        if any(not -l.blocks <= b < l.blocks for b in src_blocks):
+            raise IndexError(f"a source block is outside the pool of {l.blocks}")
+        runs = kvcopy.canonicalize_block_runs([b + l.blocks if b < 0 else b for b in src_blocks], dst_pages)
         batches = []
         per_group = self.profile.consumers_per_readiness
         for group in range(self.groups):

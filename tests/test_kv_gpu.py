@@ -145,6 +145,8 @@ def test_shared_readiness_cell_is_published_after_the_last_batch():
     (66560, 9, 70, list(range(64)), None),                                  # one long run: every CTA cuts it
     (256, 3, 700, [2 * i for i in range(300)], None),                       # more runs than one launch carries
     (1024, 2, 16, [-1, 0, 5], [2, 0, 1]),                                   # a page counted from the pool's end
+    (1024, 2, 16, [14, -1, 0, 1, -3, -2], None),                            # ... with pages before and after it
+    (256, 2, 700, [2 * i for i in range(280)] + [-2, -1, 0, 1], None),      # the same, uploaded
 ])
 def test_push_of_page_runs_copies_every_byte_and_nothing_else(page_bytes, layers, blocks, src, dst):
     import aboleth_b200 as ab
@@ -168,11 +170,16 @@ def test_push_of_page_runs_copies_every_byte_and_nothing_else(page_bytes, layers
             assert torch.equal(kv.slots, want)
             assert kv.ready[1].flatten().tolist() == [epoch] * kv.groups and int(kv.ready[0].abs().sum()) == 0
             assert int(kv._arrivals.abs().sum()) == 0
-        runs = [(s, d) for i, (s, d) in enumerate(zip(src, to)) if i == 0 or (s, d) != (src[i - 1] + 1, to[i - 1] + 1)]
+        at = [s % blocks for s in src]
+        runs = [(s, d) for i, (s, d) in enumerate(zip(at, to)) if i == 0 or (s, d) != (at[i - 1] + 1, to[i - 1] + 1)]
         off = any((kv.pool[n, s].data_ptr() | kv.slots[1, n, d].data_ptr()) & 15 for n in range(layers) for s, d in runs)
         assert (kv.status.tolist()[0] == 3) == off
-        for bad in ([blocks], [-blocks - 1]):
+        for bad in ([blocks], [-blocks - 1], [blocks - 1, blocks], [2 * i for i in range(280)] + [blocks - 1, blocks]):
+            if len(bad) > pages + 1:
+                continue
             with pytest.raises(IndexError):
                 kv.start_transfer("r", consumer=0, src_blocks=bad, slot=1, epoch=3)
         with pytest.raises(ValueError):
             kv.start_transfer("r", consumer=0, src_blocks=[], slot=1, epoch=3)
+        with pytest.raises(ValueError):
+            kv.start_transfer("r", consumer=0, src_blocks=[0, 1], slot=1, epoch=3, dst_pages=[-1, 0])

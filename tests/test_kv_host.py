@@ -41,3 +41,25 @@ def test_batches_that_publish_one_cell_share_one_arrival_counter():
     # one cell per batch degenerates to the per-batch count
     group_of, target, groups = kvcopy.pack_groups([1, 2, 3], workers=4, device="cpu")
     assert groups == 3 and group_of.tolist() == [0, 1, 2] and target.tolist() == [4, 4, 4]
+
+
+@pytest.mark.parametrize("src,dst,refused", [([7, 8], [0, 1], -4), ([6, 7, 8, 9], [0, 1, 2, 3], -4), ([8], [0], -4),
+                                             ([-9], [0], -4), ([-1, 0, 8], [0, 1, 2], -4), ([0, 1], [-1, 0], -5),
+                                             ([0, 1], [3, 4], -5), (list(range(7, -1, -1)) * 40 + [8], [1, 0] * 160 + [0], -3)])
+def test_every_page_of_a_transfer_lies_inside_the_pool_and_the_slot(src, dst, refused):
+    """A run that starts inside the pool of 8 pages (or the slot of 4) and leaves it is refused before anything is
+    launched, as a run that starts outside is; more runs than one launch carries are left to the uploaded path."""
+    import ctypes
+
+    from aboleth_b200.ops._kernels import call_rc
+
+    array, n = ctypes.c_longlong * len(src), len(src)
+    runs = ctypes.c_int(0)
+    rc = call_rc("ab_kv_push_pages", array(*src), array(*dst), n, 4096, 2, 8, 8 * 256, 256, 65536, 4 * 256, 131072, 8, 4,
+                 1, 4096, 4096, 4, 256, ctypes.byref(runs), 0)
+    assert rc == refused
+
+
+def test_a_block_counted_from_the_end_is_not_followed_by_the_first():
+    assert kvcopy.canonicalize_block_runs([-2, -1, 0, 1], [3, 4, 5, 6]) == [(-2, 3, 2), (0, 5, 2)]
+    assert kvcopy.canonicalize_block_runs([4, 5], [-1, 0]) == [(4, -1, 1), (5, 0, 1)]
