@@ -61,7 +61,10 @@ class CompiledKVTransferManager:
             world.region("kv_ready", reg, offset=pool_bytes + slot_bytes, length=cells * 8)], tag=tag)
         self.status = torch.zeros(2, dtype=torch.int64, device=world.torch_device)
         self.ledger = TransferLedger(l.slots)
-        self._arrivals = torch.zeros(4096, dtype=torch.int32, device=world.torch_device)
+        # One counter per readiness cell that this rank publishes: transfers to different slots or consumers may be in
+        # flight on different streams, and a counter that two of them shared would publish a cell too early or never.
+        self._arrivals = torch.zeros(ranks, l.slots, self.groups, dtype=torch.int32, device=world.torch_device)
+        self._counters = [consumer.unbind() for consumer in self._arrivals]
         self.last_transfer_us: Optional[float] = None
 
     # -- producer side ---------------------------------------------------------------------
@@ -75,18 +78,20 @@ class CompiledKVTransferManager:
             raise ValueError("the transfer does not fit the consumer's slot")
         if len(src_blocks) == 0:
             raise ValueError("a transfer needs at least one block")
+        if not 0 <= slot < l.slots:
+            raise IndexError(f"slot {slot} is outside the {l.slots} slots")
+        arrivals = self._counters[consumer][slot]
         slots_base = self.table.host_addresses("kv_slots")[consumer]
         ready_base = self.table.host_addresses("kv_ready")[consumer]
         ranks = self.world.world_size
         slot_base = slots_base + slot * l.layers * l.slot_layer_bytes
-        if self.groups <= self._arrivals.numel():
-            found = kvcopy.push_pages(
-                src_blocks, dst_pages, pool=self.pool, slots=slot_base, slot_layer=l.slot_layer_bytes,
-                cells=ready_base + (slot * self.groups * ranks + rank) * 8, cell_stride=ranks * 8,
-                per_group=self.profile.consumers_per_readiness, epoch=epoch, arrivals=self._arrivals,
-                status=self.status, workers=self.profile.copy_workers, threads=self.profile.threads)
-            if found is not None:
-                return found * l.layers
+        found = kvcopy.push_pages(
+            src_blocks, dst_pages, pool=self.pool, slots=slot_base, slot_layer=l.slot_layer_bytes,
+            cells=ready_base + (slot * self.groups * ranks + rank) * 8, cell_stride=ranks * 8,
+            per_group=self.profile.consumers_per_readiness, epoch=epoch, arrivals=arrivals,
+            status=self.status, workers=self.profile.copy_workers, threads=self.profile.threads)
+        if found is not None:
+            return found * l.layers
         # More runs than one launch's arguments hold: one batch per (run, layer), uploaded.
         if any(not -l.blocks <= b < l.blocks for b in src_blocks):
             raise IndexError(f"a source block is outside the pool of {l.blocks}")
@@ -106,11 +111,8 @@ class CompiledKVTransferManager:
         # batch, never by a batch that merely finished first.
         dev = self.world.torch_device
         packed = kvcopy.pack_batches(batches, dev)
-        group_of, group_target, groups = kvcopy.pack_groups([b[3] for b in batches],
-                                                            self.profile.copy_workers, dev)
-        if groups > self._arrivals.numel():
-            self._arrivals = torch.zeros(groups, dtype=torch.int32, device=dev)
-        kvcopy.push(packed, self._arrivals, len(batches), epoch, workers=self.profile.copy_workers,
+        group_of, group_target, _ = kvcopy.pack_groups([b[3] for b in batches], self.profile.copy_workers, dev)
+        kvcopy.push(packed, arrivals, len(batches), epoch, workers=self.profile.copy_workers,
                     threads=self.profile.threads, status=self.status, group_of=group_of,
                     group_target=group_target)
         launched = len(batches)

@@ -183,3 +183,28 @@ def test_push_of_page_runs_copies_every_byte_and_nothing_else(page_bytes, layers
             kv.start_transfer("r", consumer=0, src_blocks=[], slot=1, epoch=3)
         with pytest.raises(ValueError):
             kv.start_transfer("r", consumer=0, src_blocks=[0, 1], slot=1, epoch=3, dst_pages=[-1, 0])
+
+
+def test_transfers_on_two_streams_publish_their_own_cells():
+    """Transfers to two slots at the same time, each from a stream of its own, many times over: every cell shows its own
+    transfer's epoch, every byte has arrived, and the counters are zero again."""
+    import aboleth_b200 as ab
+    from aboleth_b200.kv import CompiledKVTransferManager, KVPoolLayout
+
+    torch.cuda.set_device(0)
+    with ab.World(0, 1, device=0) as world:
+        world.connect_all("p2p")
+        kv = CompiledKVTransferManager(world, KVPoolLayout(layers=8, blocks=64, page_bytes=4096, slots=2, slot_pages=32))
+        kv.pool.copy_(torch.randint(0, 255, kv.pool.shape, device="cuda", dtype=torch.uint8))
+        pages = [list(range(32)), list(range(63, 31, -1))]
+        streams = [torch.cuda.Stream() for _ in pages]
+        torch.cuda.synchronize()
+        for epoch in range(1, 21):
+            for slot, stream in enumerate(streams):
+                with torch.cuda.stream(stream):
+                    kv.start_transfer("r", consumer=0, src_blocks=pages[slot], slot=slot, epoch=epoch)
+        torch.cuda.synchronize()
+        for slot in range(2):
+            assert torch.equal(kv.slots[slot], kv.pool[:, pages[slot]])
+        assert kv.ready.flatten().tolist() == [20] * kv.ready.numel() and int(kv._arrivals.abs().sum()) == 0
+        assert kv.status.tolist()[0] == 0

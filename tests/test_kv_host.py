@@ -63,3 +63,27 @@ def test_every_page_of_a_transfer_lies_inside_the_pool_and_the_slot(src, dst, re
 def test_a_block_counted_from_the_end_is_not_followed_by_the_first():
     assert kvcopy.canonicalize_block_runs([-2, -1, 0, 1], [3, 4, 5, 6]) == [(-2, 3, 2), (0, 5, 2)]
     assert kvcopy.canonicalize_block_runs([4, 5], [-1, 0]) == [(4, -1, 1), (5, 0, 1)]
+
+
+@pytest.mark.parametrize("pages", [list(range(8)), list(range(0, 600, 2))])   # one launch's arguments, and uploaded
+def test_transfers_to_different_slots_share_no_arrival_counter(pages, monkeypatch):
+    """Each transfer counts the arrivals of its readiness groups on counters of its own: several may be in flight, also
+    on different streams, and a shared one would mix their counts."""
+    import aboleth_b200 as ab
+    from aboleth_b200.kv import CompiledKVTransferManager, KVPoolLayout
+
+    used = []
+    push_pages = lambda src, dst, *, arrivals, **_: used.append(arrivals) or (1 if len(src) == 8 else None)  # noqa: E731
+    monkeypatch.setattr(kvcopy, "push_pages", push_pages)
+    monkeypatch.setattr(kvcopy, "push", lambda packed, arrivals, *a, **k: used.append(arrivals))
+    with ab.World(0, 1, device="cpu") as world:
+        world.connect_all("p2p")
+        kv = CompiledKVTransferManager(world, KVPoolLayout(layers=9, blocks=600, page_bytes=16, slots=3, slot_pages=300))
+        for slot in range(3):
+            kv.start_transfer("r", consumer=0, src_blocks=pages, slot=slot, epoch=1)
+        counters = {a.data_ptr() + 4 * i for a in used for i in range(a.numel())}
+        assert all(a.numel() == kv.groups and a.is_contiguous() for a in used)
+        assert len(counters) == 3 * kv.groups
+        for slot in (-1, 3):
+            with pytest.raises(IndexError):
+                kv.start_transfer("r", consumer=0, src_blocks=pages, slot=slot, epoch=1)
