@@ -73,15 +73,16 @@ __device__ __forceinline__ bool mbar_try_wait(std::uint64_t *bar, unsigned parit
 }
 
 // Wait for the phase with `parity` to complete.  Gives up after ~4 s of
-// %globaltimer and reports false; the caller must then stop issuing work,
-// record the failure and fall through to its teardown.
-__device__ __forceinline__ bool mbar_wait(std::uint64_t *bar, unsigned parity) {
+// %globaltimer, or soon after another role has raised `stop`, and reports false;
+// the caller must then stop issuing work, record the failure and fall through to
+// its teardown.
+__device__ __forceinline__ bool mbar_wait(std::uint64_t *bar, unsigned parity, const volatile int *stop = nullptr) {
     for (int i = 0; i < 4096; ++i)
         if (mbar_try_wait(bar, parity))
             return true;
     const std::uint64_t start = aboleth::detail::globaltimer_ns();
     while (!mbar_try_wait(bar, parity)) {
-        if (aboleth::detail::globaltimer_ns() - start > 4000000000ull)
+        if (aboleth::detail::globaltimer_ns() - start > 4000000000ull || (stop != nullptr && *stop != 0))
             return false;
     }
     return true;

@@ -110,7 +110,7 @@ __device__ __forceinline__ void gemm_mx_mainloop_pair(Policy &policy, const Maps
         int stage = 0;
         unsigned phase = 0;
         Tile t;
-        for (int it = 0; !st.abort && policy.next(it, t); ++it) {
+        for (int it = 0; !warp_aborted(st.abort) && policy.next(it, t); ++it) {
             if (!__all_sync(0xffffffffu, !elected || policy.ready(t))) {
                 raise_abort(st, rank);
                 set_status(status, aboleth::Status::Timeout, 0x3000 + t.tag);
@@ -124,7 +124,7 @@ __device__ __forceinline__ void gemm_mx_mainloop_pair(Policy &policy, const Maps
             }
             int sfa = a_row / BM * k_blocks_a, sfb = t.b_row / 64;
             for (int kb = 0; kb < t.k_blocks; ++kb) {
-                if (!warp_wait(&st.empty[stage], phase ^ 1)) {
+                if (!warp_wait(&st.empty[stage], phase ^ 1, &st.abort)) {
                     raise_abort(st, rank);
                     set_status(status, aboleth::Status::Timeout, 0x3100 + stage);
                     break;
@@ -156,18 +156,18 @@ __device__ __forceinline__ void gemm_mx_mainloop_pair(Policy &policy, const Maps
             int stage = 0;
             unsigned phase = 0;
             Tile t;
-            for (int it = 0; !st.abort && policy.next(it, t); ++it) {
+            for (int it = 0; !warp_aborted(st.abort) && policy.next(it, t); ++it) {
                 const int slot = it & 1;
                 const std::uint32_t d = tmem_base + slot * G::kSlot1;
                 // Both CTAs' epilogues have read the columns that this tile shares with the one before.
-                if (it > 0 && !__all_sync(0xffffffffu, pair_wait(&st.tmem_empty[0], (it - 1) & 1))) {
+                if (it > 0 && !__all_sync(0xffffffffu, pair_wait(&st.tmem_empty[0], (it - 1) & 1, &st.abort))) {
                     raise_abort(st, rank);
                     set_status(status, aboleth::Status::Timeout, 0x3200 + slot);
                     break;
                 }
                 tc_fence_after();
                 for (int kb = 0; kb < t.k_blocks; ++kb) {
-                    if (!warp_wait(&st.full[stage], phase)) {
+                    if (!warp_wait(&st.full[stage], phase, &st.abort)) {
                         raise_abort(st, rank);
                         set_status(status, aboleth::Status::Timeout, 0x3300 + stage);
                         break;
@@ -226,7 +226,7 @@ __device__ __forceinline__ void gemm_mx_mainloop_pair(Policy &policy, const Maps
             if ((aborted = epilogue_aborted()))
                 break;
             const int slot = it & 1;
-            if (!mbar_wait(&st.tmem_full[slot], (it >> 1) & 1)) {
+            if (!warp_wait(&st.tmem_full[slot], (it >> 1) & 1, &st.abort)) {
                 raise_abort(st, rank);
                 set_status(status, aboleth::Status::Timeout, 0x3400 + slot);
             } else {
@@ -254,7 +254,7 @@ __device__ __forceinline__ void gemm_mx_mainloop_pair(Policy &policy, const Maps
 
     // ---------------- teardown ----------------
     __syncwarp();
-    if (st.abort) {
+    if (warp_aborted(st.abort)) {
         const std::uint64_t t0 = aboleth::detail::globaltimer_ns();
         while (aboleth::detail::globaltimer_ns() - t0 < 2000000ull)
             __nanosleep(1000);

@@ -217,7 +217,7 @@ __device__ __forceinline__ void gemm_mx_mainloop(Policy &policy, const CUtensorM
         int stage = 0;
         unsigned phase = 0;
         Tile t;
-        for (int it = 0; !st.abort && policy.next(it, t); ++it) {
+        for (int it = 0; !warp_aborted(st.abort) && policy.next(it, t); ++it) {
             if (!__all_sync(0xffffffffu, !elected || policy.ready(t))) {
                 st.abort = 1;
                 set_status(status, aboleth::Status::Timeout, 0x3000 + t.tag);
@@ -234,7 +234,7 @@ __device__ __forceinline__ void gemm_mx_mainloop(Policy &policy, const CUtensorM
                 sfb_next = static_cast<std::size_t>((t.b_row2 - t.b_row) / 64) * kAtomBytes;
             const std::size_t sfa_half = static_cast<std::size_t>(sf.k_blocks) * kAtomBytes;
             for (int kb = 0; kb < t.k_blocks; ++kb) {
-                if (!warp_wait(&st.empty[stage], phase ^ 1)) {
+                if (!warp_wait(&st.empty[stage], phase ^ 1, &st.abort)) {
                     st.abort = 1;
                     set_status(status, aboleth::Status::Timeout, 0x3100 + stage);
                     break;
@@ -274,16 +274,16 @@ __device__ __forceinline__ void gemm_mx_mainloop(Policy &policy, const CUtensorM
         int stage = 0;
         unsigned phase = 0;
         Tile t;
-        for (int it = 0; !st.abort && policy.next(it, t); ++it) {
+        for (int it = 0; !warp_aborted(st.abort) && policy.next(it, t); ++it) {
             // The accumulator must have been drained by the epilogue of the tile before.
-            if (!warp_wait(&st.tmem_empty[0], (it & 1) ^ 1)) {
+            if (!warp_wait(&st.tmem_empty[0], (it & 1) ^ 1, &st.abort)) {
                 st.abort = 1;
                 set_status(status, aboleth::Status::Timeout, 0x3200);
                 break;
             }
             tc_fence_after();
             for (int kb = 0; kb < t.k_blocks; ++kb) {
-                if (!warp_wait(&st.full[stage], phase)) {
+                if (!warp_wait(&st.full[stage], phase, &st.abort)) {
                     st.abort = 1;
                     set_status(status, aboleth::Status::Timeout, 0x3300 + stage);
                     break;
@@ -355,7 +355,7 @@ __device__ __forceinline__ void gemm_mx_mainloop(Policy &policy, const CUtensorM
                         break;
                 }
             }
-            if (!mbar_wait(&st.tmem_full[0], it & 1)) {
+            if (!warp_wait(&st.tmem_full[0], it & 1, &st.abort)) {
                 st.abort = 1;
                 set_status(status, aboleth::Status::Timeout, 0x3400);
             } else {
@@ -393,7 +393,7 @@ __device__ __forceinline__ void gemm_mx_mainloop(Policy &policy, const CUtensorM
 
     // ---------------- teardown ----------------
     __syncwarp();
-    if (st.abort) {
+    if (warp_aborted(st.abort)) {
         // Let copies that are still in flight land before the CTA's shared memory is handed on.
         const std::uint64_t t0 = aboleth::detail::globaltimer_ns();
         while (aboleth::detail::globaltimer_ns() - t0 < 2000000ull)

@@ -171,13 +171,13 @@ __device__ __forceinline__ bool pair_try_wait(std::uint64_t *bar, unsigned parit
     return ok != 0;
 }
 
-__device__ __forceinline__ bool pair_wait(std::uint64_t *bar, unsigned parity) {
+__device__ __forceinline__ bool pair_wait(std::uint64_t *bar, unsigned parity, const volatile int *abort) {
     for (int i = 0; i < 4096; ++i)
         if (pair_try_wait(bar, parity))
             return true;
     const std::uint64_t start = aboleth::detail::globaltimer_ns();
     while (!pair_try_wait(bar, parity)) {
-        if (aboleth::detail::globaltimer_ns() - start > 4000000000ull)
+        if (aboleth::detail::globaltimer_ns() - start > 4000000000ull || *abort != 0)
             return false;
     }
     return true;
@@ -237,7 +237,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtenso
         unsigned phase = 0;
         Tile t;
         AB_TRACE(long long t_wait = 0, t_begin = clock64();)
-        for (int it = 0; !st.abort && policy.next(it, t); ++it) {
+        for (int it = 0; !warp_aborted(st.abort) && policy.next(it, t); ++it) {
             if (!__all_sync(0xffffffffu, !elected || policy.ready(t))) {
                 raise_abort(st, rank);
                 set_status(status, aboleth::Status::Timeout, 0x3000 + t.tag);
@@ -250,7 +250,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtenso
                 b_row = leader ? t.b_row : t.b_row2;
             for (int kb = 0; kb < t.k_blocks; ++kb) {
                 AB_TRACE(const long long w0 = clock64();)
-                const bool got = warp_wait(&st.empty[stage], phase ^ 1);
+                const bool got = warp_wait(&st.empty[stage], phase ^ 1, &st.abort);
                 AB_TRACE(t_wait += clock64() - w0;)
                 if (!got) {
                     raise_abort(st, rank);
@@ -287,12 +287,12 @@ __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtenso
             unsigned phase = 0;
             Tile t;
             AB_TRACE(long long t_full = 0, t_acc = 0, t_begin = clock64();)
-            for (int it = 0; !st.abort && policy.next(it, t); ++it) {
+            for (int it = 0; !warp_aborted(st.abort) && policy.next(it, t); ++it) {
                 const unsigned use = use_of(it);
                 const int slot = slot_of(it);
                 for (int kb = 0; kb < t.k_blocks; ++kb) {
                     AB_TRACE(const long long f0 = clock64();)
-                    const bool filled = warp_wait(&st.full[stage], phase);
+                    const bool filled = warp_wait(&st.full[stage], phase, &st.abort);
                     AB_TRACE(t_full += clock64() - f0;)
                     if (!filled) {
                         raise_abort(st, rank);
@@ -305,7 +305,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtenso
                     if (kb == 0) {
                         // Both CTAs' epilogues must have drained this accumulator.
                         AB_TRACE(const long long a0 = clock64();)
-                        const bool free_acc = __all_sync(0xffffffffu, pair_wait(&st.tmem_empty[slot], use ^ 1));
+                        const bool free_acc = __all_sync(0xffffffffu, pair_wait(&st.tmem_empty[slot], use ^ 1, &st.abort));
                         AB_TRACE(t_acc += clock64() - a0;)
                         if (!free_acc) {
                             raise_abort(st, rank);
@@ -372,7 +372,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtenso
                         break;
                 }
             }
-            if (!mbar_wait(&st.tmem_full[slot], use)) {
+            if (!warp_wait(&st.tmem_full[slot], use, &st.abort)) {
                 raise_abort(st, rank);
                 set_status(status, aboleth::Status::Timeout, 0x3400 + slot);
             } else {
@@ -407,7 +407,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtenso
 
     // ---------------- teardown ----------------
     __syncwarp();
-    if (st.abort) {
+    if (warp_aborted(st.abort)) {
         const std::uint64_t t0 = aboleth::detail::globaltimer_ns();
         while (aboleth::detail::globaltimer_ns() - t0 < 2000000ull)
             __nanosleep(1000);

@@ -12,9 +12,9 @@
 // global -> shared by TMA (cp.async.bulk.tensor, 128-byte swizzle, never
 // multicast) through a 4-stage ring of 48 KiB stages.
 //
-// Every wait is bounded.  A role that gives up sets the CTA's abort flag; all
-// roles then leave their loops, the CTA lets copies in flight land, frees its
-// TMEM and returns with Status::Timeout recorded.
+// Every wait is bounded.  A role that gives up sets the CTA's abort flag; the other
+// roles see it in their own waits or at their next tile and leave their loops, the CTA
+// lets copies in flight land, frees its TMEM and returns with Status::Timeout recorded.
 #pragma once
 
 #include <cuda.h>
@@ -60,9 +60,15 @@ __device__ __forceinline__ bool elect_one() {
     return pred != 0;
 }
 
-// A whole warp waits and takes one way out, also where the wait runs out for some lanes only.
-__device__ __forceinline__ bool warp_wait(std::uint64_t *bar, unsigned parity) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+// A whole warp waits and takes one way out, also where the wait runs out, or sees `abort`, for some lanes only.
+__device__ __forceinline__ bool warp_wait(std::uint64_t *bar, unsigned parity, const volatile int *abort) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort));
+}
+
+// The abort flag as a whole warp takes it: other warps, and the pair's other CTA, raise it at any time, so lanes
+// that read it one by one could see different values, and the ones that stay would wait for the others for good.
+__device__ __forceinline__ bool warp_aborted(const volatile int &abort) {
+    return __any_sync(0xffffffffu, abort != 0);
 }
 
 // ---- tcgen05 wrappers --------------------------------------------------------------
@@ -398,7 +404,7 @@ __device__ __forceinline__ void gemm_mainloop(Policy &policy, const CUtensorMap 
         int stage = 0;
         unsigned phase = 0;
         Tile t;
-        for (int it = 0; !st.abort && policy.next(it, t); ++it) {
+        for (int it = 0; !warp_aborted(st.abort) && policy.next(it, t); ++it) {
             if (!__all_sync(0xffffffffu, !elected || policy.ready(t))) {
                 st.abort = 1;
                 set_status(status, aboleth::Status::Timeout, 0x3000 + t.tag);
@@ -406,7 +412,7 @@ __device__ __forceinline__ void gemm_mainloop(Policy &policy, const CUtensorMap 
             }
             const CUtensorMap *tile_map_a = t.a_sel ? map_a_alt : map_a;
             for (int kb = 0; kb < t.k_blocks; ++kb) {
-                if (!warp_wait(&st.empty[stage], phase ^ 1)) {
+                if (!warp_wait(&st.empty[stage], phase ^ 1, &st.abort)) {
                     st.abort = 1;
                     set_status(status, aboleth::Status::Timeout, 0x3100 + stage);
                     break;
@@ -438,10 +444,10 @@ __device__ __forceinline__ void gemm_mainloop(Policy &policy, const CUtensorMap 
         int stage = 0;
         unsigned phase = 0;
         Tile t;
-        for (int it = 0; !st.abort && policy.next(it, t); ++it) {
+        for (int it = 0; !warp_aborted(st.abort) && policy.next(it, t); ++it) {
             const unsigned use = use_of(it);
             for (int kb = 0; kb < t.k_blocks; ++kb) {
-                if (!warp_wait(&st.full[stage], phase)) {
+                if (!warp_wait(&st.full[stage], phase, &st.abort)) {
                     st.abort = 1;
                     set_status(status, aboleth::Status::Timeout, 0x3300 + stage);
                     break;
@@ -455,7 +461,7 @@ __device__ __forceinline__ void gemm_mainloop(Policy &policy, const CUtensorMap 
                     const int slot = slot_of(it, h);
                     if (kb == 0) {
                         // The accumulator must have been drained by the epilogue.
-                        if (!warp_wait(&st.tmem_empty[slot], use ^ 1)) {
+                        if (!warp_wait(&st.tmem_empty[slot], use ^ 1, &st.abort)) {
                             drained = false;
                             st.abort = 1;
                             set_status(status, aboleth::Status::Timeout, 0x3200 + slot);
@@ -531,7 +537,7 @@ __device__ __forceinline__ void gemm_mainloop(Policy &policy, const CUtensorMap 
                             break;
                     }
                 }
-                if (!mbar_wait(&st.tmem_full[slot], use)) {
+                if (!warp_wait(&st.tmem_full[slot], use, &st.abort)) {
                     st.abort = 1;
                     set_status(status, aboleth::Status::Timeout, 0x3400 + slot);
                     break;
@@ -569,7 +575,7 @@ __device__ __forceinline__ void gemm_mainloop(Policy &policy, const CUtensorMap 
 
     // ---------------- teardown ----------------
     __syncwarp();
-    if (st.abort) {
+    if (warp_aborted(st.abort)) {
         // Let TMA copies that are still in flight land before the CTA's shared
         // memory is handed to another CTA.
         const std::uint64_t t0 = aboleth::detail::globaltimer_ns();

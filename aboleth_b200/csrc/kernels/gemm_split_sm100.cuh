@@ -149,7 +149,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         int stage = 0;
         unsigned phase = 0;
         for (int kb = kb0; kb < kb1; ++kb) {
-            if (!warp_wait(&st.empty[stage], phase ^ 1)) {
+            if (!warp_wait(&st.empty[stage], phase ^ 1, &st.abort)) {
                 st.abort = 1;
                 set_status(p.status, aboleth::Status::Timeout, 0x3700 + stage);
                 break;
@@ -181,7 +181,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         int stage = 0;
         unsigned phase = 0;
         for (int kb = kb0; kb < kb1; ++kb) {
-            if (!warp_wait(&st.full[stage], phase)) {
+            if (!warp_wait(&st.full[stage], phase, &st.abort)) {
                 st.abort = 1;
                 set_status(p.status, aboleth::Status::Timeout, 0x3720 + stage);
                 break;
@@ -219,7 +219,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     } else {
         // TMEM lane = weight row, column = token: the partial tile goes to shared memory as [token][weight row],
         // over the stages, which every MMA has read by now.
-        if (!warp_wait(&st.done, 0)) {
+        if (!warp_wait(&st.done, 0, &st.abort)) {
             st.abort = 1;
             set_status(p.status, aboleth::Status::Timeout, 0x3740);
         } else {
@@ -239,7 +239,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         }
     }
     __syncwarp();
-    if (st.abort) {
+    if (warp_aborted(st.abort)) {
         // Let copies that are still in flight land before the shared memory is handed on.
         const std::uint64_t t0 = aboleth::detail::globaltimer_ns();
         while (aboleth::detail::globaltimer_ns() - t0 < 2000000ull)

@@ -135,3 +135,40 @@ def test_gemm_reduce_scatter_block_scaled_e4m3(world, m_local, k_local, n):
         group.rs[r].check()
         want = total[r * m_local:(r + 1) * m_local].to(torch.bfloat16)
         assert torch.equal(outs[r], want)
+
+
+@pytest.mark.parametrize("kind", ["bf16", "mx"])
+def test_a_shard_that_never_arrives_ends_every_role_at_the_first_limit(kind):
+    """Rank 1 never pushes: the producer's wait for its chunk runs out (2 s), and the issuer and the epilogue, which
+    wait up to 4 s for operands and accumulators, leave with it.  The own rows are there, and the device works on."""
+    from aboleth_b200.parallel import LocalTpGroup
+    from aboleth_b200.parallel.tp import CONSUME, PRODUCE
+
+    world, m_local, k, n = 2, 256, 256, 256
+    g = torch.Generator(device="cuda").manual_seed(3)
+    ranks = [_mx_operands(m_local, n, k, g) for _ in range(world)]
+    group = LocalTpGroup(world, m_local, k, 256)
+    op = group.ag[0]
+    if kind == "mx":
+        run, args, full = op.mx, ranks[0][0], [r[1] for r in ranks] + [ranks[0][2]]
+    else:
+        full = [torch.randn(m_local, k, generator=g, device="cuda").to(torch.bfloat16) for _ in range(3)]
+        run, args = op, (full[0], full[2])
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    out = run(*args, phases=PRODUCE)
+    torch.cuda.synchronize()
+    start.record()
+    out = run(*args, out, phases=CONSUME, advance=False)
+    end.record()
+    torch.cuda.synchronize()
+    assert op.status.tolist() == [1, 0x3001]
+    assert 1900 < start.elapsed_time(end) < 3000
+    assert _rel(out[:m_local], full[0].float() @ full[2].float().t()) < 5e-3
+    again = LocalTpGroup(world, m_local, k, 256)
+    if kind == "mx":
+        outs = again.ag_gemm_mx(*[[r[0][i] for r in ranks] for i in range(4)])
+    else:
+        outs = again.ag_gemm(full[:2], [full[2]] * 2)
+    torch.cuda.synchronize()
+    again.ag[0].check()
+    assert _rel(outs[0], torch.cat(full[:2]).float() @ full[2].float().t()) < 5e-3
