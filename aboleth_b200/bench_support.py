@@ -156,8 +156,9 @@ class EpLayerBench:
         bad = int((~(err <= tol)).sum().item())  # NaN rows count as errors
         return bad
 
-    def _traffic(self) -> dict:
-        """Bytes this rank moved in the last step (records it sent / got back)."""
+    def _traffic(self, weighted: bool) -> dict:
+        """Bytes this rank moved in the last step (records it sent / got back).  ``weighted``: the combine gathers a
+        record's rows, one per choice."""
         s, slot = self.spec, self.layer.slot
         slots = slot.source_slots[: self.tokens]
         sent = (slots >= 0).sum(dim=0).tolist()
@@ -167,9 +168,9 @@ class EpLayerBench:
         return {"records_total": total, "records_remote": remote,
                 "dispatch_remote_bytes": remote * record, "combine_remote_bytes": remote * s.hidden * 2,
                 "dispatch_local_hbm_bytes": self.tokens * s.hidden * 2 + total * record,
-                # one rank writes a token's result straight from its record: no return segment
-                "combine_local_hbm_bytes": total * s.hidden * 2 * (1 if s.ranks == 1 else 2) +
-                                           self.tokens * s.hidden * 2}
+                # the expert rows in; the return segment out and in, which one rank does not have; the result out
+                "combine_local_hbm_bytes": (total * ((s.top_k if weighted else 1) + (0 if s.ranks == 1 else 2)) +
+                                            self.tokens) * s.hidden * 2}
 
     def phase_times(self, *, steps: int, distributed: bool, flush: bool = False,
                     weighted: Optional[bool] = None) -> dict:
@@ -226,7 +227,7 @@ class EpLayerBench:
         torch.cuda.synchronize()
         kernel_trace["combine"] = slot.trace()
         slot.trace_buffer = None
-        traffic = self._traffic()
+        traffic = self._traffic(weighted)
         peaks = measured_peaks()
         roof = {"traffic": traffic, "denominators": peaks["source"]}
         if self.world.world_size > 1:

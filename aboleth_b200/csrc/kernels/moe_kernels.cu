@@ -1262,17 +1262,24 @@ __global__ void __launch_bounds__(kThreads, 3) ep_combine_kernel(const __grid_co
 // (4096 tokens x hidden 7168, top-8: 95 us, 24 warps 103; two of four 117, one of eight 144, the general kernel
 // 126), one piece of eight rows where a part is a single piece (128 tokens: 7 us, the general kernel 16).  The sums are taken in the order, and rounded to bf16 at the
 // places, of the general kernel (whose second pass adds a lone partial to zero).
-template <bool WEIGHTED, int kPieces>
-__global__ void __launch_bounds__(kThreads, kPieces == 4 ? 4 : 3) ep_combine_local_kernel(const __grid_constant__ CombineParams p, int parts) {
+template <bool WEIGHTED, int kPieces, bool TRACED = false>
+__global__ void __launch_bounds__(kThreads, kPieces == 4 ? 4 : 3)
+ep_combine_local_kernel(const __grid_constant__ CombineParams p, int parts) {
     const EpGeometry &g = p.g;
     const int lane = threadIdx.x & 31;
     const int vecs = g.hidden / 8, groups = (vecs + 31) / 32;
+    if constexpr (TRACED)
+        stamp(p.trace, 0, blockIdx.x == 0 && threadIdx.x == 0);
     if (blockIdx.x == 0 && threadIdx.x == 0)
         *p.epoch += 1;  // no CTA of this launch reads it
     const long long item = static_cast<long long>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
     const int t = static_cast<int>(item / parts), part = static_cast<int>(item - static_cast<long long>(t) * parts);
-    if (t >= p.num_tokens)
+    if (t >= p.num_tokens) {
+        if constexpr (TRACED)  // a layer without tokens
+            for (int i = 1; i <= 4; ++i)
+                stamp(p.trace, i, item == 0 && lane == 0);
         return;
+    }
     const int slot = p.source_slots[t];
     std::uint32_t *out = p.out + static_cast<std::size_t>(t) * (g.hidden / 2);
     const int first = part * groups / parts * 32, last = min((part + 1) * groups / parts * 32, vecs);
@@ -1330,6 +1337,14 @@ __global__ void __launch_bounds__(kThreads, kPieces == 4 ? 4 : 3) ep_combine_loc
                 *reinterpret_cast<uint4 *>(out + v * 4) = pack_bf16x8(sum);
         }
     }
+    if constexpr (TRACED)
+        if (lane == 0) {  // the first item is sent and reduced at once; the last warp ends the layer
+            const unsigned long long now = aboleth::detail::globaltimer_ns();
+            if (item == 0)
+                p.trace[1] = p.trace[2] = now;
+            atomicMax(p.trace + 3, now);
+            atomicMax(p.trace + 4, now);
+        }
 }
 
 // ---- standalone pieces ------------------------------------------------------------
@@ -1614,7 +1629,10 @@ bool geometry_ok(const EpGeometry &g) {
 
 // CTAs of the last dispatch (0) / combine (1) launch made by the calling host thread.
 static thread_local int g_last_grid[2] = {0, 0};
-AB_EXPORT int ab_ep_last_grid(int which) { return which == 0 || which == 1 ? g_last_grid[which] : -1; }
+static thread_local bool g_last_local[2] = {false, false};
+AB_EXPORT int ab_ep_last_grid(int which) {
+    return which == 0 || which == 1 ? g_last_grid[which] | (g_last_local[which] ? 1 << 30 : 0) : -1;
+}
 
 // Argument blocks are passed as arrays of 64-bit words so the Python side needs
 // no struct mirror: ints[] carries the integer geometry, ptrs[] the addresses.
@@ -1695,6 +1713,7 @@ AB_EXPORT int ab_ep_dispatch(const int *ints, float amax_floor, const std::uint6
                                        : resident_grid<ep_dispatch_local_kernel<false>>(1 << 30);
         grid = std::max(1, std::min(requested > 0 ? requested : p.num_tokens, held));
         g_last_grid[0] = grid;
+        g_last_local[0] = true;
         if (p.g.value_fp8)
             ep_dispatch_local_kernel<true><<<grid, kThreads, 0, stream>>>(p);
         else
@@ -1702,6 +1721,7 @@ AB_EXPORT int ab_ep_dispatch(const int *ints, float amax_floor, const std::uint6
         return ab::launch_result("ep_dispatch");
     }
     g_last_grid[0] = grid;
+    g_last_local[0] = false;
     if (p.by_warp)
         ep_dispatch_kernel<true><<<grid, kThreads, 0, stream>>>(p);
     else
@@ -1752,7 +1772,7 @@ AB_EXPORT int ab_ep_combine(const int *ints, float amax_floor, const std::uint64
     p.trace = reinterpret_cast<unsigned long long *>(ptrs[i++]);
     if (p.weighted && p.expert_offsets == nullptr)
         return -1;
-    if (p.g.world == 1 && p.phases == (kPhaseSend | kPhaseRecv) && p.trace == nullptr) {
+    if (p.g.world == 1 && p.phases == (kPhaseSend | kPhaseRecv)) {
         // Enough (token, part) items for every warp the device holds; a part has at least 512 bytes on the
         // latency path and 2 KiB on the throughput path (what keeps DRAM pages open).
         const int groups = (p.g.hidden / 8 + 31) / 32, finest = p.by_warp ? (groups + 3) / 4 : groups;
@@ -1760,12 +1780,19 @@ AB_EXPORT int ab_ep_combine(const int *ints, float amax_floor, const std::uint64
         const int parts = std::max(1, std::min(finest, p.num_tokens > 0 ? (wanted + p.num_tokens - 1) / p.num_tokens : 1));
         const long long items = static_cast<long long>(p.num_tokens) * parts;
         g_last_grid[1] = static_cast<int>(std::max(1LL, (items + kWarps - 1) / kWarps));
-        const auto kernel = !p.weighted ? ep_combine_local_kernel<false, 8>
-                            : parts * 2 > groups ? ep_combine_local_kernel<true, 1> : ep_combine_local_kernel<true, 4>;
+        g_last_local[1] = true;
+        const bool short_parts = parts * 2 > groups;
+        const auto kernel =
+            p.trace == nullptr ? (!p.weighted ? ep_combine_local_kernel<false, 8>
+                                  : short_parts ? ep_combine_local_kernel<true, 1> : ep_combine_local_kernel<true, 4>)
+                               : (!p.weighted ? ep_combine_local_kernel<false, 8, true>
+                                  : short_parts ? ep_combine_local_kernel<true, 1, true>
+                                                : ep_combine_local_kernel<true, 4, true>);
         kernel<<<g_last_grid[1], kThreads, 0, stream>>>(p, parts);
         return ab::launch_result("ep_combine");
     }
     g_last_grid[1] = resident_grid<ep_combine_kernel>(grid);
+    g_last_local[1] = false;
     ep_combine_kernel<<<g_last_grid[1], kThreads, 0, stream>>>(p);
     return ab::launch_result("ep_combine");
 }

@@ -128,9 +128,11 @@ class DispatchResult:
 declare("ab_ep_last_grid", [ctypes.c_int])
 
 
-def _last_grid(which: int) -> int:
-    """CTAs of the last dispatch (0) or combine (1) launch of this thread."""
-    return lib().ab_ep_last_grid(which)
+def _last_launch(which: int) -> tuple[int, str]:
+    """CTAs of the last dispatch (0) or combine (1) launch of this thread, and which kernel it was.  The one for a
+    world of one rank takes no notice of ``by_warp`` (dispatch), ``send_warps`` and ``return_block``."""
+    got = lib().ab_ep_last_grid(which)
+    return got & ~(1 << 30), "one rank" if got >> 30 & 1 else "general"
 
 
 class MoEBuffers:
@@ -320,7 +322,7 @@ class NativeMoESlot:
         pointers[28] = ptr(self.trace_buffer)
         call("ab_ep_dispatch", self._geometry(n, routing, renormalize, phases), s.quant_amax_floor, pointers,
              self.grid, stream_ptr())
-        self.last_launch["grid"] = _last_grid(0)
+        self.last_launch["grid"], self.last_launch["kernel"] = _last_launch(0)
         self.launched["dispatch"] = self.last_launch
         self._last_tokens = n
         return DispatchResult(self.recv_payload, self.expert_scales, self.expert_ids,
@@ -361,7 +363,7 @@ class NativeMoESlot:
         pointers[17] = ptr(self.trace_buffer)
         call("ab_ep_combine", self._geometry(n, 0, False, phases, int(expert_offsets is not None)),
              s.quant_amax_floor, pointers, self.grid, stream_ptr())
-        self.last_launch["grid"] = _last_grid(1)
+        self.last_launch["grid"], self.last_launch["kernel"] = _last_launch(1)
         self.last_launch["weighted"] = expert_offsets is not None
         self.launched["combine"] = self.last_launch
         return out[:n]
@@ -376,7 +378,8 @@ class NativeMoESlot:
         Dispatch: ``first_cta_sent``, ``all_sent`` (the last CTA arrived and publishes),
         ``peers_seen`` (every peer's flag observed), ``end``.  Combine: ``first_cta_sent``,
         ``first_cta_reduced``, ``all_reduced`` (last CTA arrived), ``end`` (every peer said it
-        finished sending)."""
+        finished sending).  With one rank a token is sent and reduced by the same warp: the combine's first
+        two stamps are its first item's end, the last two the last one's."""
         t = self.trace_buffer.tolist()
         us = lambda b: (t[b] - t[0]) / 1e3 if t[0] and t[b] else None  # noqa: E731
         return {"first_cta_sent": us(1), "all_sent_or_first_reduced": us(2), "peers_seen_or_all_reduced": us(3),

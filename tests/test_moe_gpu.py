@@ -282,3 +282,39 @@ def test_one_rank_launches_equal_the_general_ones(fp8, tokens, hidden, experts, 
             got.append(records + [out, plain])
         for a, b in zip(*got):
             assert torch.equal(torch.nan_to_num(a.float()), torch.nan_to_num(b.float()))
+
+
+@pytest.mark.parametrize("tokens", [0, 1, 130])
+def test_one_rank_trace_describes_the_kernels_that_run_without_it(tokens):
+    """Tracing neither changes which kernel runs nor its grid nor its result, and the stamps are in order."""
+    from aboleth_b200.moe.native import LocalMoEGroup
+    from aboleth_b200.moe.spec import MoESpec
+    from aboleth_b200.ops import expert_offsets, standin_expert
+
+    spec = MoESpec(capacity=130, hidden=1024, top_k=4, experts=16, ranks=1)
+    slot = LocalMoEGroup(spec).slots[0]
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn(tokens, 1024, generator=g, device="cuda").to(torch.bfloat16)
+    logits = torch.randn(tokens, 16, generator=g, device="cuda")
+    outs, launched, stamps = [], [], []
+    for traced in (False, True):
+        if traced:
+            slot.enable_trace()
+        res = slot.dispatch(x, logits=logits)
+        if traced:
+            stamps.append(slot.trace())
+            slot.trace_buffer.zero_()
+        offsets, _ = expert_offsets(res.expert_counts_by_source)
+        rows = torch.zeros(130 * 4, 1024, dtype=torch.bfloat16, device="cuda")
+        standin_expert(res.expert_input, res.expert_scales, rows, res.expert_ids, res.expert_weights, res.expert_pos,
+                       res.recv_counts, world=1, capacity=130, group=128, offsets=offsets)
+        outs.append(slot.combine(rows, expert_offsets=offsets).clone())
+        if traced:
+            stamps.append(slot.trace())
+        launched.append({k: dict(v) for k, v in slot.launched.items()})
+    slot.check()
+    assert launched[0] == launched[1] and launched[0]["combine"]["kernel"] == launched[0]["dispatch"]["kernel"] == "one rank"
+    assert torch.equal(outs[0], outs[1])
+    for stamp in stamps:
+        assert all(v is not None for v in stamp.values()), stamp
+        assert list(stamp.values()) == sorted(stamp.values())
