@@ -145,7 +145,7 @@ __device__ __forceinline__ void warp_softmax_topk_n(const Logit *logits, int exp
 #pragma unroll
     for (int i = 0; i < PER_LANE; ++i) {
         sum += (lane + 32 * i) < experts ? __expf(v[i] - mx) : 0.f;
-        const std::uint32_t raw = __float_as_uint(v[i]);
+        const std::uint32_t raw = __float_as_uint(v[i] + 0.0f);  // -0 becomes 0: equal logits have equal keys
         key[i] = v[i] > -INFINITY ? raw ^ ((raw >> 31) ? 0xffffffffu : 0x80000000u) : 0u;
     }
     for (int off = 16; off > 0; off >>= 1)

@@ -318,3 +318,24 @@ def test_one_rank_trace_describes_the_kernels_that_run_without_it(tokens):
     for stamp in stamps:
         assert all(v is not None for v in stamp.values()), stamp
         assert list(stamp.values()) == sorted(stamp.values())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("experts", [8, 40, 96, 256, 320])
+def test_router_takes_equal_logits_in_index_order_whatever_their_zeros_sign(experts, dtype):
+    """0.0 and -0.0 are equal: the lower index is chosen first, also where both lie in one lane (32 experts apart)."""
+    from aboleth_b200.ops import router_topk
+
+    g = torch.Generator(device="cuda").manual_seed(experts)
+    logits = torch.randint(-1, 2, (64, experts), generator=g, device="cuda").to(dtype)
+    logits = torch.where((logits == 0) & (torch.rand(64, experts, generator=g, device="cuda") < 0.5), -logits.abs(), logits)
+    logits[0] = -0.0
+    logits[1] = 0.0
+    logits[0, 3:5] = 0.0
+    logits[1, 0:3] = -0.0
+    ids, weights = router_topk(logits, 8)
+    torch.cuda.synchronize()
+    want = torch.sort(logits.float(), dim=-1, descending=True, stable=True)
+    assert torch.equal(ids.long(), want.indices[:, :8])
+    # the fast exponential: a few 2^-22
+    assert torch.allclose(weights, torch.softmax(logits.float(), -1).gather(1, want.indices[:, :8]), rtol=1e-5, atol=0)
