@@ -179,7 +179,10 @@ class MixtralEP:
     def moe_layer(self, x: torch.Tensor, layer: dict) -> torch.Tensor:
         c = self.config
         tokens = x.shape[0]
-        ids, weights = router_topk(x @ layer["router"].t(), c.top_k, renormalize=True)
+        logits = x @ layer["router"].t()
+        if logits.dtype != torch.bfloat16:  # under autocast the product is what that asks for
+            logits = logits.float()
+        ids, weights = router_topk(logits, c.top_k, renormalize=True)
         if self.fp8_experts:
             return self._moe_layer_fp8(x, layer, ids, weights)
         prepared = self.moe.prepare(x, weights, ids, with_local_counts=False)

@@ -97,3 +97,28 @@ def test_fp8_experts_run_block_scaled_end_to_end():
         model.check()
         check_gemm_status("cuda")
         assert out.shape == (4, 3)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+def test_moe_layer_under_half_precision_autocast(fp8):
+    """Autocast makes the router's product fp16 (or fp32): the layer takes such logits as it takes bf16 ones."""
+    import aboleth_b200 as ab
+    from aboleth_b200.models import MixtralConfig, MixtralEP
+
+    cfg = MixtralConfig(layers=1, hidden=256, experts=4, top_k=2, ffn=512, heads=4, kv_heads=2, vocab=128, max_seq=64)
+    with ab.World(0, 1, device=0) as world:
+        world.connect_all("p2p")
+        model = MixtralEP(cfg, world, max_batch=4, max_prompt=16, seed=3, fp8_experts=fp8)
+        g = torch.Generator(device="cuda").manual_seed(1)
+        x = torch.randn(37, 256, generator=g, device="cuda").to(torch.bfloat16)
+        layer = model.layers[0]
+        ordered = torch.sort((x @ layer["router"].t()).float(), dim=-1, descending=True).values
+        clear = ordered[:, 1] - ordered[:, 2] > 0.05   # no rounding of the logits moves the choice of these tokens
+        with torch.no_grad():
+            want = model.moe_layer(x, layer).float()
+            with torch.autocast("cuda", dtype=torch.float16):
+                got = model.moe_layer(x, layer).float()
+        torch.cuda.synchronize()
+        model.check()
+        assert int(clear.sum()) > 10
+        assert ((got - want)[clear].norm() / want[clear].norm()).item() < 2e-2
