@@ -11,6 +11,7 @@
 // kernels is cuBLAS through torch.matmul.
 #include <algorithm>
 #include <atomic>
+#include <cstdlib>
 
 #include "gemm_mx_pair_sm100.cuh"
 #include "gemm_mx_sm100.cuh"
@@ -562,8 +563,17 @@ struct DenseChoice {
     int nt, split;   // nt <= 0: a persistent loop, of `split` CTAs per tile (-1: with 224 columns a tile)
 };
 
+// What an environment variable asks for, or -1.
+int asked(const char *name) {
+    const char *v = std::getenv(name);
+    return v == nullptr || *v == 0 ? -1 : std::atoi(v);
+}
+
+// ABOLETH_GEMM_PAIR: 0 = no CTA pairs (the split kernel), 1 or 2 = CTA pairs, for bf16 and per-tensor e4m3.
+// ABOLETH_GEMM_MX_TILE: 1 = 128 x 256 tiles of one CTA, 2 = 256 x 256 tiles of a pair, for block-scaled e4m3.
 template <typename Op>
 DenseChoice choose_dense(int m, int n, int k_blocks, int kind) {
+    const int forced = asked(kind == kKindMx ? "ABOLETH_GEMM_MX_TILE" : "ABOLETH_GEMM_PAIR");
     struct Row { int nt; double lone, packed; };
     static const Row kDense[4] = {{32, .213, .278}, {64, .251, .365}, {128, .278, .482}, {256, .336, .336}};
     static const Row kScaled[4] = {{32, .263, .586}, {64, .473, .473}, {128, .324, .564}, {256, .306, .306}};
@@ -592,6 +602,12 @@ DenseChoice choose_dense(int m, int n, int k_blocks, int kind) {
             best_us = one;
             best = DenseChoice{0, 1};
         }
+        if (forced > 0)
+            return DenseChoice{0, forced == 1 ? 1 : 2};
+    } else if (forced > 0) {
+        return best;
+    } else if (forced == 0) {
+        best_us = 1e30;
     }
     for (int i = 0; i < 4; ++i) {
         const int nt = rows[i].nt;
@@ -622,6 +638,24 @@ DenseChoice choose_dense(int m, int n, int k_blocks, int kind) {
     }
     return best;
 }
+
+}  // namespace
+
+// Which kernel a dense product of this size takes: choice[0] > 0 - the split kernel with that token tile and K in
+// choice[1] parts; 0 or -1 - a persistent loop over tiles of choice[1] CTAs, 256 or 224 columns wide.
+AB_EXPORT int ab_gemm_choice(int kind, int m, int n, int k, int *choice) {
+    if (kind < kKindBf16 || kind > kKindMx || m < 1 || n < 1 || k < 1 || choice == nullptr)
+        return -1;
+    const int k_blocks = kind == kKindBf16 ? (k + 63) / 64 : (k + 127) / 128;
+    const DenseChoice c = kind == kKindBf16 ? choose_dense<OpBf16>(m, n, k_blocks, kind)
+                          : kind == kKindE4m3 ? choose_dense<OpE4m3>(m, n, k_blocks, kind)
+                                              : choose_dense<split::OpMx>(m, n, k_blocks, kind);
+    choice[0] = c.nt;
+    choice[1] = c.split;
+    return 0;
+}
+
+namespace {
 
 template <typename Op>
 int launch_dense(const DenseArgs &d, int kind, cudaStream_t stream) {

@@ -105,3 +105,21 @@ def test_connection_info_version_skew():
         abi.ConnectionInfo.from_bytes(bytes(info))
     with pytest.raises(ValueError, match="128 bytes"):
         abi.ConnectionInfo.from_bytes(b"\0" * 64)
+
+
+def test_packed_scale_sizes_are_those_of_the_library():
+    """The size of the packed scales is worked out in Python, where buffers are made, and in the library, whose kernels
+    index them: a difference would be an access out of range."""
+    import ctypes
+
+    from aboleth_b200.ops._kernels import lib
+    from aboleth_b200.ops.gemm import _mx_scale_bytes, mx_scale_bytes
+
+    native = lib().ab_mx_scale_bytes
+    native.restype, native.argtypes = ctypes.c_longlong, [ctypes.c_int] * 4
+    for m in (1, 127, 128, 129, 255, 4096, 4097):
+        for n in (1, 8, 63, 64, 65, 128, 200, 8192):
+            for k in (1, 127, 128, 129, 7168):
+                for which in (0, 1):
+                    assert _mx_scale_bytes(m, n, k, which) == native(m, n, k, which), (m, n, k, which)
+                assert mx_scale_bytes(m, k) == native(m, n, k, 0)

@@ -152,9 +152,11 @@ def test_block_scaled_e4m3_gemm_matches_fp32(m, n, k, pow2):
     assert torch.equal(dequant_block_scaled(wide[:, :k], a_s), a_deq)
 
 
-@pytest.mark.parametrize("tile,m,n,k", [("1", 300, 640, 512),     # 128 x 256 tiles: partial rows, 2.5 column tiles
-                                         ("2", 300, 640, 512),     # 256 x 192 tiles: tiles start at odd granules
-                                         ("2", 700, 1000, 384)])   # three row tiles, ragged last column tile
+@pytest.mark.parametrize("tile,m,n,k", [("1", 300, 640, 512),     # one CTA: partial rows, 2.5 column tiles
+                                         ("2", 300, 640, 512),     # CTA pairs: a second row tile of 44 rows
+                                         ("2", 700, 1000, 384),    # three row tiles, ragged last column tile
+                                         ("1", 3000, 5000, 128),   # several tiles per CTA, one K step
+                                         ("2", 3000, 5000, 128)])  # ... and per pair: both accumulators, in turn
 def test_block_scaled_mx_gemm_is_exact_on_integers_and_flags_bad_scales(tile, m, n, k, monkeypatch):
     """Small integers and power-of-two scales: every product and partial sum is exact, so the
     tensor-core path must reproduce the fp32 result bit for bit (after the bf16 rounding of the
@@ -178,7 +180,7 @@ def test_block_scaled_mx_gemm_is_exact_on_integers_and_flags_bad_scales(tile, m,
     assert torch.equal(out, want)
     # a scale that is not a power of two cannot be carried as ue8m0: reported, not silently rounded
     bad = a_s.clone()
-    bad[5, 1] = 0.3
+    bad[5, -1] = 0.3
     gemm_e4m3_block_scaled(a_q, bad, b_q, b_s)
     torch.cuda.synchronize()
     assert gemm_status(out.device)[:2].tolist() == [3, 0x3500]
@@ -218,7 +220,8 @@ def test_grouped_block_scaled_gemm_is_exact_on_integers(counts):
 
 
 @pytest.mark.parametrize("counts,n,k", [([0, 5, 128, 200, 1, 131], 320, 264),    # 128-row tiles, 2.5 column tiles
-                                        ([700, 0, 1031, 517], 1288, 192)])      # 256-row tiles, ragged columns
+                                        ([700, 0, 1031, 517], 1288, 192),       # 256-row tiles, ragged columns
+                                        ([1000, 1281, 897, 640], 2048, 64)])    # 256 of them on 74 pairs, one K step
 def test_grouped_swiglu_gemm_matches_fp32(counts, n, k):
     """silu(a gate^T) * (a up^T) per expert.  The oracle is fp32 over the same bf16 operands, so what differs
     is the one bf16 rounding of the result (2^-9 relative, 1.7e-3 in the mean) and the fast exponential (a few
@@ -245,7 +248,8 @@ def test_grouped_swiglu_gemm_matches_fp32(counts, n, k):
         assert bool((out[lo + cnt:lo + int(padded[e])] == 7.0).all())  # rows outside the expert are never written
 
 
-@pytest.mark.parametrize("counts,n,k", [([0, 5, 128, 200, 1, 131], 384, 384), ([700, 0, 300], 128, 128)])
+@pytest.mark.parametrize("counts,n,k", [([0, 5, 128, 200, 1, 131], 384, 384), ([700, 0, 300], 128, 128),
+                                        ([1000, 1281, 897, 640], 2048, 128)])   # 256 pair tiles on 74 pairs
 def test_grouped_swiglu_block_scaled_gemm_is_its_parts(counts, n, k):
     """The fused gate / up product and its quantisation against the separate passes: block-scaled product, SiLU and
     multiply in bf16, ``quant_fp8``.  Both round to bf16 at the same three places; only the exponential differs, by a
@@ -282,6 +286,112 @@ def test_grouped_swiglu_block_scaled_gemm_is_its_parts(counts, n, k):
     assert bool((q[~live].float() == 7.0).all()) and bool((by_row(packed)[~live] == 0).all())
     assert torch.equal(by_row(packed)[live], by_row(want_packed)[live])
     assert float((q[live].float() != want[live].float()).double().mean()) <= 2.0 ** -11
+
+
+def _dense(kind, a, b, out, g):
+    """The public entry point of a kind on small integers; the fp32 operands that it stands for."""
+    from aboleth_b200.ops import gemm_bf16, gemm_e4m3, gemm_e4m3_mx, pack_scales_mx
+
+    (m, k), n = a.shape, b.shape[0]
+    if kind == "bf16":
+        gemm_bf16(a.bfloat16(), b.bfloat16(), out)
+        return a, b
+    fp8 = torch.float8_e4m3fn
+    if kind == "e4m3":
+        gemm_e4m3(a.to(fp8), b.to(fp8), out)
+        return a, b
+    a_s = torch.exp2(torch.randint(-2, 3, (m, k // 128), generator=g, device="cuda").float())
+    b_s = torch.exp2(torch.randint(-2, 3, (-(-n // 128), k // 128), generator=g, device="cuda").float())
+    gemm_e4m3_mx(a.to(fp8), pack_scales_mx(a_s, m, k, weight=False), b.to(fp8), pack_scales_mx(b_s, n, k, weight=True),
+                 out)
+    return (a * a_s.repeat_interleave(128, dim=1),
+            b * b_s.repeat_interleave(128, dim=0)[:n].repeat_interleave(128, dim=1))
+
+
+def _dense_case(kind, m, n, k):
+    from aboleth_b200.ops import check_gemm_status
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randint(-2, 3, (m, k), generator=g, device="cuda").float()
+    b = torch.randint(-2, 3, (n, k), generator=g, device="cuda").float()
+    wide = torch.full((m + 1, n + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    a_full, b_full = _dense(kind, a, b, wide[:m, :n], g)
+    torch.cuda.synchronize()
+    check_gemm_status("cuda")
+    assert torch.equal(wide[:m, :n], (a_full @ b_full.t()).to(torch.bfloat16))
+    assert bool((wide[m] == 7.0).all()) and bool((wide[:, n:] == 7.0).all())
+
+
+def _choice(kind, m, n, k):
+    import ctypes
+
+    from aboleth_b200.ops._kernels import call
+
+    choice = (ctypes.c_int * 2)()
+    call("ab_gemm_choice", ("bf16", "e4m3", "mx").index(kind), m, n, k, choice)
+    return choice[0], choice[1]
+
+
+# The kernels of the dispatch: a token tile of the split kernel; a loop with 256- (0) or 224-column (-1) pair tiles;
+# for block-scaled operands the one-CTA loop (0, 1) and the pair loop (0, 2).
+@pytest.mark.parametrize("kind,m,n,k,kernel", [
+    ("bf16", 1, 312, 256, 32), ("bf16", 232, 2664, 256, 64), ("bf16", 132, 3872, 2048, 128),
+    ("bf16", 2649, 1584, 1024, 256), ("bf16", 587, 5448, 384, 0), ("bf16", 227, 4840, 256, -1),
+    ("e4m3", 1, 280, 256, 32), ("e4m3", 65, 6968, 256, 64), ("e4m3", 303, 1832, 3840, 128),
+    ("e4m3", 783, 4624, 2176, 256), ("e4m3", 1920, 2112, 256, 0), ("e4m3", 1676, 704, 256, -1),
+    ("mx", 1, 256, 256, 32), ("mx", 56, 288, 768, 64), ("mx", 129, 3296, 2304, 128), ("mx", 2721, 1544, 1024, 256),
+    ("mx", 75, 360, 256, (0, 1)), ("mx", 905, 8136, 1024, (0, 2))])
+def test_dense_gemm_through_every_kernel_of_its_dispatch(kind, m, n, k, kernel):
+    """One size per outcome of the rule that picks the kernel, exact on integers, in a strided output."""
+    choice = _choice(kind, m, n, k)
+    assert (choice if isinstance(kernel, tuple) else choice[0]) == kernel
+    _dense_case(kind, m, n, k)
+
+
+@pytest.mark.parametrize("kind", ["bf16", "e4m3"])
+@pytest.mark.parametrize("m,n,k,width", [(3000, 5000, 64, 224), (3000, 5000, 320, 224), (9470, 1504, 64, 256)])
+def test_pair_loop_with_several_tiles_per_pair(kind, m, n, k, width, monkeypatch):
+    """More than two tiles for every pair, so that both accumulators are used again, with one K step (the issuer
+    runs ahead of the epilogue) and a few; the switch asks for pairs where the rule would not."""
+    monkeypatch.setenv("ABOLETH_GEMM_PAIR", "1")
+    assert _choice(kind, m, n, k) == (0 if width == 256 else -1, 2)
+    assert -(-m // 256) * -(-n // width) > 2 * 74
+    _dense_case(kind, m, n, k)
+    monkeypatch.setenv("ABOLETH_GEMM_PAIR", "0")
+    assert _choice(kind, m, n, k)[0] > 0
+    _dense_case(kind, m, n, k)
+
+
+@pytest.mark.parametrize("k", [128, 384])
+def test_grouped_pair_loops_with_several_tiles_per_pair(k):
+    """The same for the grouped products: 17 row tiles x 16 column tiles on 74 pairs, ragged last row tiles."""
+    from aboleth_b200.ops import check_gemm_status, grouped_gemm_bf16, grouped_gemm_e4m3_mx, pack_scales_mx
+
+    n, fp8 = 4096, torch.float8_e4m3fn
+    counts = torch.tensor([1000, 1281, 897, 640], dtype=torch.int32, device="cuda")
+    tiles = int(((counts + 255) // 256).sum()) * n // 256
+    assert tiles > 3 * 74
+    padded = (counts + 127) // 128 * 128
+    offsets = (torch.cumsum(padded, 0) - padded).to(torch.int32)
+    rows = int(padded.sum())
+    g = torch.Generator(device="cuda").manual_seed(k)
+    a = torch.randint(-2, 3, (rows, k), generator=g, device="cuda").float()
+    w = torch.randint(-2, 3, (4, n, k), generator=g, device="cuda").float()
+    a_s = torch.exp2(torch.randint(-2, 3, (rows, k // 128), generator=g, device="cuda").float())
+    w_s = torch.exp2(torch.randint(-2, 3, (4, n // 128, k // 128), generator=g, device="cuda").float())
+    plain = grouped_gemm_bf16(a.bfloat16(), w.bfloat16(), counts, offsets)
+    scaled = torch.full((rows, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    grouped_gemm_e4m3_mx(a.to(fp8), pack_scales_mx(a_s, rows, k, weight=False), w.to(fp8),
+                         pack_scales_mx(w_s.view(-1, k // 128), 4 * n, k, weight=True), counts, offsets, scaled)
+    torch.cuda.synchronize()
+    check_gemm_status("cuda")
+    a_full = a * a_s.repeat_interleave(128, dim=1)
+    for e in range(4):
+        live = slice(int(offsets[e]), int(offsets[e]) + int(counts[e]))
+        w_full = w[e] * w_s[e].repeat_interleave(128, dim=0).repeat_interleave(128, dim=1)
+        assert torch.equal(plain[live], (a[live] @ w[e].t()).to(torch.bfloat16))
+        assert torch.equal(scaled[live], (a_full[live] @ w_full.t()).to(torch.bfloat16))
+        assert bool((scaled[live.stop:int(offsets[e]) + int(padded[e])] == 7.0).all())
 
 
 def _split_case(kind, m, n, k, nt, split):
@@ -326,7 +436,7 @@ def test_split_gemm_is_exact_on_integers_for_every_tile_and_split(kind, m, n, k)
 @pytest.mark.parametrize("kind", ["bf16", "e4m3"])
 @pytest.mark.parametrize("m", [1, 31, 32, 33, 64, 65, 128, 129, 256, 257, 700, 1500])
 def test_dense_gemm_agrees_across_its_dispatch(kind, m):
-    """Row counts on both sides of every boundary of the rule that picks the kernel, in a strided output."""
+    """Row counts around the edges of the token tiles, in a strided output."""
     from aboleth_b200.ops import check_gemm_status, gemm_bf16, gemm_e4m3
 
     n, k = 1160, 1040
@@ -345,8 +455,7 @@ def test_dense_gemm_agrees_across_its_dispatch(kind, m):
 @pytest.mark.parametrize("n", [128, 640])
 def test_grouped_pair_tiles_at_their_edges(counts, n):
     """Experts just over and under a 256-row pair tile, one with a single row, one column tile that is half full:
-    small integers are exact in both operand types, and the two accumulators of the block-scaled loop share columns,
-    so several tiles in a row have to come out right."""
+    small integers are exact in both operand types.  (At most one tile per pair here.)"""
     from aboleth_b200.ops import check_gemm_status, grouped_gemm_bf16, grouped_gemm_e4m3_mx, pack_scales_mx
 
     experts, k = len(counts), 256
@@ -394,9 +503,9 @@ def test_pair_tiles_of_both_widths_are_exact_on_integers(m, n, k):
 
 
 def test_chained_launches_see_what_the_kernels_before_them_wrote():
-    """Quantise, pack and multiply in a row, with nothing waiting in between, over buffers that the next round overwrites:
-    the results are those of the same calls with a synchronisation after each, also when the chain is captured in a graph
-    and when another stream runs one at the same time."""
+    """Quantise, pack and multiply in a row, with nothing waiting in between, over buffers that the next round
+    overwrites: the results are those of the same calls with a synchronisation after each, also when the chain is captured
+    in a graph and when another stream runs one at the same time."""
     from aboleth_b200.ops import gemm_bf16, gemm_e4m3_mx, pack_scales_mx, quant_fp8
 
     m, n, k = 257, 640, 512

@@ -194,7 +194,8 @@ def test_transfers_on_two_streams_publish_their_own_cells():
     torch.cuda.set_device(0)
     with ab.World(0, 1, device=0) as world:
         world.connect_all("p2p")
-        kv = CompiledKVTransferManager(world, KVPoolLayout(layers=8, blocks=64, page_bytes=4096, slots=2, slot_pages=32))
+        layout = KVPoolLayout(layers=8, blocks=64, page_bytes=4096, slots=2, slot_pages=32)
+        kv = CompiledKVTransferManager(world, layout)
         kv.pool.copy_(torch.randint(0, 255, kv.pool.shape, device="cuda", dtype=torch.uint8))
         pages = [list(range(32)), list(range(63, 31, -1))]
         streams = [torch.cuda.Stream() for _ in pages]

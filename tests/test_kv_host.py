@@ -45,7 +45,8 @@ def test_batches_that_publish_one_cell_share_one_arrival_counter():
 
 @pytest.mark.parametrize("src,dst,refused", [([7, 8], [0, 1], -4), ([6, 7, 8, 9], [0, 1, 2, 3], -4), ([8], [0], -4),
                                              ([-9], [0], -4), ([-1, 0, 8], [0, 1, 2], -4), ([0, 1], [-1, 0], -5),
-                                             ([0, 1], [3, 4], -5), (list(range(7, -1, -1)) * 40 + [8], [1, 0] * 160 + [0], -3)])
+                                             ([0, 1], [3, 4], -5),
+                                             (list(range(7, -1, -1)) * 40 + [8], [1, 0] * 160 + [0], -3)])
 def test_every_page_of_a_transfer_lies_inside_the_pool_and_the_slot(src, dst, refused):
     """A run that starts inside the pool of 8 pages (or the slot of 4) and leaves it is refused before anything is
     launched, as a run that starts outside is; more runs than one launch carries are left to the uploaded path."""
@@ -55,8 +56,8 @@ def test_every_page_of_a_transfer_lies_inside_the_pool_and_the_slot(src, dst, re
 
     array, n = ctypes.c_longlong * len(src), len(src)
     runs = ctypes.c_int(0)
-    rc = call_rc("ab_kv_push_pages", array(*src), array(*dst), n, 4096, 2, 8, 8 * 256, 256, 65536, 4 * 256, 131072, 8, 4,
-                 1, 4096, 4096, 4, 256, ctypes.byref(runs), 0)
+    rc = call_rc("ab_kv_push_pages", array(*src), array(*dst), n, 4096, 2, 8, 8 * 256, 256, 65536, 4 * 256, 131072, 8,
+                 4, 1, 4096, 4096, 4, 256, ctypes.byref(runs), 0)
     assert rc == refused
 
 
@@ -73,12 +74,17 @@ def test_transfers_to_different_slots_share_no_arrival_counter(pages, monkeypatc
     from aboleth_b200.kv import CompiledKVTransferManager, KVPoolLayout
 
     used = []
-    push_pages = lambda src, dst, *, arrivals, **_: used.append(arrivals) or (1 if len(src) == 8 else None)  # noqa: E731
+
+    def push_pages(src, dst, *, arrivals, **_):
+        used.append(arrivals)
+        return 1 if len(src) == 8 else None
+
     monkeypatch.setattr(kvcopy, "push_pages", push_pages)
     monkeypatch.setattr(kvcopy, "push", lambda packed, arrivals, *a, **k: used.append(arrivals))
     with ab.World(0, 1, device="cpu") as world:
         world.connect_all("p2p")
-        kv = CompiledKVTransferManager(world, KVPoolLayout(layers=9, blocks=600, page_bytes=16, slots=3, slot_pages=300))
+        layout = KVPoolLayout(layers=9, blocks=600, page_bytes=16, slots=3, slot_pages=300)
+        kv = CompiledKVTransferManager(world, layout)
         for slot in range(3):
             kv.start_transfer("r", consumer=0, src_blocks=pages, slot=slot, epoch=1)
         counters = {a.data_ptr() + 4 * i for a in used for i in range(a.numel())}

@@ -313,7 +313,8 @@ def test_one_rank_trace_describes_the_kernels_that_run_without_it(tokens):
             stamps.append(slot.trace())
         launched.append({k: dict(v) for k, v in slot.launched.items()})
     slot.check()
-    assert launched[0] == launched[1] and launched[0]["combine"]["kernel"] == launched[0]["dispatch"]["kernel"] == "one rank"
+    assert launched[0] == launched[1]
+    assert launched[0]["combine"]["kernel"] == launched[0]["dispatch"]["kernel"] == "one rank"
     assert torch.equal(outs[0], outs[1])
     for stamp in stamps:
         assert all(v is not None for v in stamp.values()), stamp
@@ -328,7 +329,8 @@ def test_router_takes_equal_logits_in_index_order_whatever_their_zeros_sign(expe
 
     g = torch.Generator(device="cuda").manual_seed(experts)
     logits = torch.randint(-1, 2, (64, experts), generator=g, device="cuda").to(dtype)
-    logits = torch.where((logits == 0) & (torch.rand(64, experts, generator=g, device="cuda") < 0.5), -logits.abs(), logits)
+    negative = (logits == 0) & (torch.rand(64, experts, generator=g, device="cuda") < 0.5)
+    logits = torch.where(negative, -logits.abs(), logits)
     logits[0] = -0.0
     logits[1] = 0.0
     logits[0, 3:5] = 0.0
