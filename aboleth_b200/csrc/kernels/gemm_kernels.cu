@@ -71,7 +71,8 @@ struct PlainPolicy {
 template <int CTAS, bool SWIGLU>
 struct GroupedPolicy {
     static constexpr int kRows = BM * CTAS, kCols = SWIGLU ? BN / 2 : BN;
-    static constexpr bool kBackground = false, kDrainedHook = false, kScaled = false, kSwiGlu = SWIGLU, kNarrowA = CTAS == 1;
+    static constexpr bool kBackground = false, kDrainedHook = false, kScaled = false;
+    static constexpr bool kSwiGlu = SWIGLU, kNarrowA = CTAS == 1;
     __nv_bfloat16 *c;
     const int *counts, *offsets;
     int experts, n, k, ldc, tiles_n;
@@ -257,7 +258,8 @@ struct MxPolicy {
 template <int CTAS, bool SWIGLU>
 struct GroupedMxPolicy {
     static constexpr int kRows = BM * CTAS, kCols = SWIGLU ? BN / 2 : BN;
-    static constexpr bool kBackground = false, kDrainedHook = false, kScaled = false, kSwiGlu = SWIGLU, kNarrowA = CTAS == 1;
+    static constexpr bool kBackground = false, kDrainedHook = false, kScaled = false;
+    static constexpr bool kSwiGlu = SWIGLU, kNarrowA = CTAS == 1;
     std::uint8_t *c;
     std::uint32_t *packed;
     const int *counts, *offsets;
@@ -312,7 +314,8 @@ struct GroupedMxPolicy {
     }
     __device__ __forceinline__ void store_scale(const Tile &t, int row, std::uint32_t word) const {
         const int r = t.c_row + row;
-        packed[(static_cast<std::size_t>(r / BM) * (n / 128) + t.c_col / 128) * 128 + (r % 32) * 4 + (r % BM) / 32] = word;
+        const std::size_t atom = static_cast<std::size_t>(r / BM) * (n / 128) + t.c_col / 128;
+        packed[atom * 128 + (r % 32) * 4 + (r % BM) / 32] = word;
     }
     __device__ __forceinline__ void tile_done(const Tile &) const {}
     __device__ __forceinline__ void finish(int, int, unsigned long long *) const {}
@@ -552,13 +555,13 @@ namespace {
 //     their own and `packed` beside a second CTA; at least what the slowest of the memory system needs
 //     (6.3 GB/ms from memory, 19.8 GB/ms from L2 to the SMs).
 //   pair loop: 4.6 + waves of resident pairs x (0.297 per K step + 0.45); 0.268 with 224 columns a tile, which wins
-//     where it needs no more waves (8192 x 3584 x 8192: 7 waves either way, 417 -> 375 us back to back; 8192^3: 16
-//     waves against 14, 874 and 849).
+//     where it needs no more waves (8192 x 3584 x 8192: 7 waves either way, 339 us against 449; 8192^3: 16 waves
+//     against 14, 860 and 842).
 //   block-scaled: persistent 128 x 256 tiles of one CTA, 4.2 + waves x (0.30 per K step + 1), or of a pair,
 //     5.4 + waves x (0.315 + 1), and 12.3 GB/ms of tile traffic (50 and 68 KB per tile and step).
-// bf16: 32 x 3584 x 8192 16.5 us (pair loop 42.6); 1000 x 3584 x 8192 pair loop 42.7 (split 52.8).
-// Block-scaled: 32 x 3584 x 8192 10 us (one CTA 33); 1000 x 8192 x 3584 pair loop 27.4 (one CTA 32.8, split 36);
-// 8192^3 pair loop 388 (one CTA 498); 500 x 8192 x 512 one CTA 6.7 (pair 7.9, split 8.9).
+// Back to back, launches included.  bf16: 32 x 3584 x 8192 split 17.3 us (pair loop 39.4); 1000 x 3584 x 8192 pair loop
+// 51 (256 columns 61, split 67).  Block-scaled: 32 x 3584 x 8192 split 12.3 us (one CTA 28.7); 1000 x 8192 x 3584 pair
+// loop 32.8 (one CTA 34.8); 8192^3 pair loop 452 (one CTA 499); 500 x 8192 x 512 one CTA 9.2 (pair 10.1).
 struct DenseChoice {
     int nt, split;   // nt <= 0: a persistent loop, of `split` CTAs per tile (-1: with 224 columns a tile)
 };
@@ -569,7 +572,8 @@ int asked(const char *name) {
     return v == nullptr || *v == 0 ? -1 : std::atoi(v);
 }
 
-// ABOLETH_GEMM_PAIR: 0 = no CTA pairs (the split kernel), 1 or 2 = CTA pairs, for bf16 and per-tensor e4m3.
+// ABOLETH_GEMM_PAIR: 0 = no CTA pairs (the split kernel), 1 = CTA pairs with 256 x 256 tiles, 2 = with 256 x 224
+// tiles, for bf16 and per-tensor e4m3.
 // ABOLETH_GEMM_MX_TILE: 1 = 128 x 256 tiles of one CTA, 2 = 256 x 256 tiles of a pair, for block-scaled e4m3.
 template <typename Op>
 DenseChoice choose_dense(int m, int n, int k_blocks, int kind) {
@@ -605,7 +609,7 @@ DenseChoice choose_dense(int m, int n, int k_blocks, int kind) {
         if (forced > 0)
             return DenseChoice{0, forced == 1 ? 1 : 2};
     } else if (forced > 0) {
-        return best;
+        return DenseChoice{forced == 1 ? 0 : -1, 2};
     } else if (forced == 0) {
         best_us = 1e30;
     }

@@ -19,9 +19,10 @@
 //
 // Barriers.  `full[s]` lives in the leader: both CTAs' TMA loads complete their bytes on
 // it (the peer's loads name the leader's barrier through its shared::cluster address); the
-// leader's producer makes the one arrival and announces the bytes of both.  `empty[s]`, `tmem_full[b]` exist in both CTAs and are
-// signalled by one tcgen05.commit that is multicast to the pair.  `tmem_empty[b]` lives in
-// the leader and counts the epilogue warps of both CTAs.  No TMA load is multicast.
+// leader's producer makes the one arrival and announces the bytes of both.  `empty[s]`,
+// `tmem_full[b]` exist in both CTAs and are signalled by one tcgen05.commit that is multicast
+// to the pair.  `tmem_empty[b]` lives in the leader and counts the epilogue warps of both CTAs.
+// No TMA load is multicast.
 //
 // Every wait is bounded as in the single-CTA loop; the two CTAs meet at a cluster barrier
 // before the tensor memory is freed, so neither leaves while its peer can still touch it.
@@ -58,7 +59,6 @@ struct PairState {
     std::uint64_t tmem_empty[2];        // used in the leader only
     std::uint32_t tmem_base;
     volatile int abort;
-    volatile int epi_ready;
     volatile int epi_abort;  // epilogue warps: shared sample of `abort`
 };
 
@@ -150,13 +150,6 @@ __device__ __forceinline__ void remote_arrive(std::uint32_t bar_cluster_addr) {
                  : "memory");
 }
 
-__device__ __forceinline__ void remote_arrive_expect_tx(std::uint32_t bar_cluster_addr, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(
-                     bar_cluster_addr),
-                 "r"(bytes)
-                 : "memory");
-}
-
 // A wait that also acquires, at cluster scope, what the peer CTA released.  Used once per tile
 // (the accumulator hand-back); the per-K-step waits use the CTA-scope form.
 __device__ __forceinline__ bool pair_try_wait(std::uint64_t *bar, unsigned parity) {
@@ -183,18 +176,16 @@ __device__ __forceinline__ bool pair_wait(std::uint64_t *bar, unsigned parity, c
     return true;
 }
 
-// Policy concept: the one of gemm_mainloop, with tiles of 256 rows.
+// Policy concept: the one of gemm_mainloop, with tiles of 256 rows, one A operand and no background work or drained
+// hook.
 // `policy.next` must hand the SAME tile to both CTAs of a pair (index tiles by blockIdx.x / 2
 // out of gridDim.x / 2).  Rows passed to `store16` are rows of the tile.  map_a and map_b boxes
 // are 128 and NT / 2 rows x 128 bytes; `Op` selects bf16 or e4m3 operands.
 template <typename Op, int NT, typename Policy>
 __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtensorMap *map_a,
-                                                   const CUtensorMap *map_b, unsigned long long *status,
-                                                   const CUtensorMap *map_a_alt = nullptr) {
+                                                   const CUtensorMap *map_b, unsigned long long *status) {
     using G = PairGeometry<NT>;
     constexpr int kStagesG = G::kStages;
-    if (map_a_alt == nullptr)
-        map_a_alt = map_a;
     extern __shared__ std::uint8_t smem_raw[];
     __shared__ PairState st;
     std::uint8_t *tiles = reinterpret_cast<std::uint8_t *>(
@@ -243,7 +234,6 @@ __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtenso
                 set_status(status, aboleth::Status::Timeout, 0x3000 + t.tag);
                 break;
             }
-            const CUtensorMap *tile_map_a = t.a_sel ? map_a_alt : map_a;
             const int a_row = t.a_row + static_cast<int>(rank) * G::kRowsPerCta;
             int b_row = t.b_row + static_cast<int>(rank) * (NT / 2);
             if constexpr (Policy::kSwiGlu)  // the leader brings the gate half, the peer the up half
@@ -264,7 +254,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtenso
                     // (A cluster-scope release arrive per K step cost ~1400 cycles and starved the pipe.)
                     if (leader)
                         mbar_expect_tx(&st.full[stage], 2 * G::kStageBytes);
-                    pair_tma_load_2d(sa, tile_map_a, kb * Op::kBK, a_row, full_in_leader);
+                    pair_tma_load_2d(sa, map_a, kb * Op::kBK, a_row, full_in_leader);
                     pair_tma_load_2d(sa + G::kBytesA, map_b, kb * Op::kBK, b_row, full_in_leader);
                 }
                 __syncwarp();
@@ -305,7 +295,8 @@ __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtenso
                     if (kb == 0) {
                         // Both CTAs' epilogues must have drained this accumulator.
                         AB_TRACE(const long long a0 = clock64();)
-                        const bool free_acc = __all_sync(0xffffffffu, pair_wait(&st.tmem_empty[slot], use ^ 1, &st.abort));
+                        const bool free_acc =
+                            __all_sync(0xffffffffu, pair_wait(&st.tmem_empty[slot], use ^ 1, &st.abort));
                         AB_TRACE(t_acc += clock64() - a0;)
                         if (!free_acc) {
                             raise_abort(st, rank);
@@ -361,17 +352,6 @@ __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtenso
                 break;
             const unsigned use = use_of(it);
             const int slot = slot_of(it);
-            if constexpr (Policy::kBackground) {
-                for (;;) {
-                    if (epi_thread == 0)
-                        st.epi_ready = mbar_try_wait(&st.tmem_full[slot], use) ? 1 : 0;
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
-                    const int ready_now = st.epi_ready;
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
-                    if (ready_now || !policy.background(epi_thread, kEpiThreads))
-                        break;
-                }
-            }
             if (!warp_wait(&st.tmem_full[slot], use, &st.abort)) {
                 raise_abort(st, rank);
                 set_status(status, aboleth::Status::Timeout, 0x3400 + slot);
@@ -389,17 +369,8 @@ __device__ __forceinline__ void gemm_mainloop_pair(Policy &policy, const CUtenso
                     remote_arrive(map_to_cta(smem_u32(&st.tmem_empty[slot]), 0));
             }
             asm volatile("bar.sync 1, 128;" ::: "memory");
-            if constexpr (Policy::kDrainedHook) {
-                policy.drained(t, epi_thread, kEpiThreads);
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-            }
             if (warp == 2 && lane == 0)
                 policy.tile_done(t);
-        }
-        if constexpr (Policy::kBackground) {
-            while (!aborted && !(aborted = epilogue_aborted()) &&
-                   policy.background(epi_thread, kEpiThreads)) {
-            }
         }
         if (!aborted && !epilogue_aborted())
             policy.finish(epi_thread, kEpiThreads, status);

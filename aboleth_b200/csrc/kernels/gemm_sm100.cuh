@@ -662,29 +662,4 @@ inline bool make_map_atoms(CUtensorMap *map, const void *base, std::uint64_t ato
     return rc == CUDA_SUCCESS;
 }
 
-// Convert 32 fp32 to bf16 and store 64 contiguous bytes (row-major C).
-__device__ __forceinline__ void store_row32_bf16(__nv_bfloat16 *dst, const float (&v)[32],
-                                                 int cols_left) {
-    if (cols_left >= 32 && (reinterpret_cast<std::uintptr_t>(dst) & 15) == 0) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            uint4 o;
-            __nv_bfloat162 p0 = __floats2bfloat162_rn(v[q * 8 + 0], v[q * 8 + 1]);
-            __nv_bfloat162 p1 = __floats2bfloat162_rn(v[q * 8 + 2], v[q * 8 + 3]);
-            __nv_bfloat162 p2 = __floats2bfloat162_rn(v[q * 8 + 4], v[q * 8 + 5]);
-            __nv_bfloat162 p3 = __floats2bfloat162_rn(v[q * 8 + 6], v[q * 8 + 7]);
-            o.x = *reinterpret_cast<std::uint32_t *>(&p0);
-            o.y = *reinterpret_cast<std::uint32_t *>(&p1);
-            o.z = *reinterpret_cast<std::uint32_t *>(&p2);
-            o.w = *reinterpret_cast<std::uint32_t *>(&p3);
-            *reinterpret_cast<uint4 *>(dst + q * 8) = o;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-            if (i < cols_left)
-                dst[i] = __float2bfloat16_rn(v[i]);
-    }
-}
-
 }  // namespace ab::gemm

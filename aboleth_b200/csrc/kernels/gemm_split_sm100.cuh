@@ -3,8 +3,8 @@
 //   C[M, N] = A[M, K] * B[N, K]^T,  computed tile by tile as C^T: the MMA's 128 rows are rows of B (weights),
 //   its NT columns rows of A (tokens).
 //
-// Why: the persistent pair loop gives 512 x 256 of C to two SMs.  With few tokens, or a small C, most SMs get
-// no tile and the ones that work walk the whole K alone: 32 x 3584 x 8192 took 82 us on 28 SMs, against the
+// Why: the persistent pair loop gives 256 x 256 of C to two SMs.  With few tokens, or a small C, most SMs get
+// no tile and the ones that work walk the whole K alone: 32 x 3584 x 8192 takes 43 us on 28 SMs, against the
 // 9 us its 59 MB of weights take at copy bandwidth.  Here one CTA owns 128 x NT of C^T and 1 / S of K; the S
 // CTAs of a cluster add their fp32 partial tiles through distributed shared memory, in cluster-rank order (the
 // result does not depend on timing), and each stores 1 / S of the tile.  No workspace, no second launch.
@@ -250,7 +250,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         cluster_sync();
     // Each CTA sums and stores its share of the tokens, eight weight rows (16 bytes of C) per thread.
     const int tokens = min(NT, p.m - y0);
-    const int t_begin = tokens * static_cast<int>(rank) / p.split, t_end = tokens * (static_cast<int>(rank) + 1) / p.split;
+    const int t_begin = tokens * static_cast<int>(rank) / p.split;
+    const int t_end = tokens * (static_cast<int>(rank) + 1) / p.split;
     const std::uint32_t base = smem_u32(tiles);
     for (int i = t_begin * 16 + threadIdx.x; i < t_end * 16; i += kThreads) {
         const int y = i >> 4, x = (i & 15) * 8;

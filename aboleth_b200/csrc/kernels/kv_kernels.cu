@@ -168,8 +168,9 @@ __global__ void __launch_bounds__(512, 2) kv_push_pages_kernel(const __grid_cons
     for (int group = 0, layer0 = 0; layer0 < p.layers; ++group, layer0 += p.per_group) {
         const int count = min(p.per_group, p.layers - layer0);
         const std::uint64_t total = layer_bytes * count;
-        std::uint64_t at = total / gridDim.x * blockIdx.x + total % gridDim.x * blockIdx.x / gridDim.x;
-        const std::uint64_t end = total / gridDim.x * (blockIdx.x + 1) + total % gridDim.x * (blockIdx.x + 1) / gridDim.x;
+        const std::uint64_t share = total / gridDim.x, rest = total % gridDim.x;
+        std::uint64_t at = share * blockIdx.x + rest * blockIdx.x / gridDim.x;
+        const std::uint64_t end = share * (blockIdx.x + 1) + rest * (blockIdx.x + 1) / gridDim.x;
         while (at < end) {
             // The run that byte `at` of the group lies in, and this CTA's bytes of it.  Cuts fall on 16-byte
             // boundaries of the run: the CTA before stops where this one starts.
@@ -263,7 +264,7 @@ AB_EXPORT int ab_kv_push_pages(const long long *src, const long long *dst, int p
         }
     // Two CTAs per SM, a CTA's share of a full group at least one round of its threads' loads, and no more CTAs
     // than the profile's workers per batch allow.
-    const std::uint64_t group_bytes = page_bytes * pages * static_cast<std::uint64_t>(layers < per_group ? layers : per_group);
+    const std::uint64_t group_bytes = page_bytes * pages * ab::min64(layers, per_group);
     const std::uint64_t round = static_cast<std::uint64_t>(threads) * 16 * 2;
     std::uint64_t grid = (group_bytes + round - 1) / round;
     grid = ab::min64(grid, 296);

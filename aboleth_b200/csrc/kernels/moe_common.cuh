@@ -114,6 +114,9 @@ __device__ __forceinline__ float group_max(float v, int width) {
     return v;
 }
 
+__device__ __forceinline__ float logit_of(float v) { return v; }
+__device__ __forceinline__ float logit_of(__nv_bfloat16 v) { return __bfloat162float(v); }
+
 // One warp: softmax over `experts` logits and the `top_k` largest, ties to
 // the lower index.  Lane l holds experts l, l+32, ...  On return lane j < top_k
 // holds (id, weight) of the j-th choice.  `renormalize` divides the selected
@@ -123,9 +126,6 @@ __device__ __forceinline__ float group_max(float v, int width) {
 // choose - a NaN, minus infinity, or taken), a lane's largest key comes from a tree of integer maxima, and the
 // lowest index that holds the warp's largest key from a second one; weights are computed once, after the rounds.
 // (Floating-point compares in a chain, and a weight per round, made routing most of a decode-size dispatch.)
-__device__ __forceinline__ float logit_of(float v) { return v; }
-__device__ __forceinline__ float logit_of(__nv_bfloat16 v) { return __bfloat162float(v); }
-
 template <int PER_LANE, typename Logit>
 __device__ __forceinline__ void warp_softmax_topk_n(const Logit *logits, int experts, int top_k,
                                                     int renormalize, int &out_id, float &out_w) {

@@ -1260,8 +1260,9 @@ __global__ void __launch_bounds__(kThreads, 3) ep_combine_kernel(const __grid_co
 // still fills the device.  Reading the expert rows is what bounds it: eight 16-byte loads per lane in flight, from
 // kRows rows in kPieces consecutive 512-byte pieces - four pieces of two rows and 32 warps per SM for long parts
 // (4096 tokens x hidden 7168, top-8: 95 us, 24 warps 103; two of four 117, one of eight 144, the general kernel
-// 126), one piece of eight rows where a part is a single piece (128 tokens: 7 us, the general kernel 16).  The sums are taken in the order, and rounded to bf16 at the
-// places, of the general kernel (whose second pass adds a lone partial to zero).
+// 126), one piece of eight rows where a part is a single piece (128 tokens: 7 us, the general kernel 16).  The sums
+// are taken in the order, and rounded to bf16 at the places, of the general kernel (whose second pass adds a lone
+// partial to zero).
 template <bool WEIGHTED, int kPieces, bool TRACED = false>
 __global__ void __launch_bounds__(kThreads, kPieces == 4 ? 4 : 3)
 ep_combine_local_kernel(const __grid_constant__ CombineParams p, int parts) {
@@ -1465,11 +1466,12 @@ __global__ void __launch_bounds__(kThreads) permute_kernel(
                 d[v] = s[v];
             if (dst_packed != nullptr)
                 for (int c = threadIdx.x; c < cols; c += kThreads) {
-                    const unsigned bits = __float_as_uint(src_scales[static_cast<std::size_t>(row) * src_scale_stride + c]);
+                    const float scale = src_scales[static_cast<std::size_t>(row) * src_scale_stride + c];
+                    const unsigned bits = __float_as_uint(scale);
                     if ((bits & 0x807fffffu) != 0 || (bits >> 23) == 0 || (bits >> 23) == 255)
                         ab::set_status(status, Status::Malformed, 0x3500);
-                    dst_packed[(static_cast<std::size_t>(out / 128) * cols + c) * 128 + (out % 32) * 4 + (out % 128) / 32] =
-                        ((bits >> 23) & 0xffu) * 0x01010101u;
+                    const std::size_t atom = static_cast<std::size_t>(out / 128) * cols + c;
+                    dst_packed[atom * 128 + (out % 32) * 4 + (out % 128) / 32] = ((bits >> 23) & 0xffu) * 0x01010101u;
                 }
             else if (src_scales != nullptr)
                 for (int c = threadIdx.x; c < cols; c += kThreads)
@@ -1777,7 +1779,8 @@ AB_EXPORT int ab_ep_combine(const int *ints, float amax_floor, const std::uint64
         // latency path and 2 KiB on the throughput path (what keeps DRAM pages open).
         const int groups = (p.g.hidden / 8 + 31) / 32, finest = p.by_warp ? (groups + 3) / 4 : groups;
         const int wanted = resident_grid<ep_combine_local_kernel<true, 4>>(1 << 30) * kWarps;
-        const int parts = std::max(1, std::min(finest, p.num_tokens > 0 ? (wanted + p.num_tokens - 1) / p.num_tokens : 1));
+        const int each = p.num_tokens > 0 ? (wanted + p.num_tokens - 1) / p.num_tokens : 1;
+        const int parts = std::max(1, std::min(finest, each));
         const long long items = static_cast<long long>(p.num_tokens) * parts;
         g_last_grid[1] = static_cast<int>(std::max(1LL, (items + kWarps - 1) / kWarps));
         g_last_local[1] = true;
@@ -1840,9 +1843,10 @@ AB_EXPORT int ab_expert_offsets(const int *counts, int *offsets, int *total, int
 }
 
 static int launch_permute(const void *src, void *dst, const float *src_scales, float *dst_scales, const int *expert_ids,
-                          const int *expert_pos, const int *offsets, const unsigned long long *recv_counts, int *perm_row,
-                          int world, int capacity, int top_k, int row_bytes, int cols, int src_scale_stride,
-                          int offset_stride, void *dst_packed, unsigned long long *status, cudaStream_t stream) {
+                          const int *expert_pos, const int *offsets, const unsigned long long *recv_counts,
+                          int *perm_row, int world, int capacity, int top_k, int row_bytes, int cols,
+                          int src_scale_stride, int offset_stride, void *dst_packed, unsigned long long *status,
+                          cudaStream_t stream) {
     if (row_bytes % 16 || world < 1 || capacity < 1)
         return -1;
     const int total = world * capacity;
@@ -1850,7 +1854,8 @@ static int launch_permute(const void *src, void *dst, const float *src_scales, f
     permute_kernel<<<grid, kThreads, 0, stream>>>(
         static_cast<const std::uint8_t *>(src), static_cast<std::uint8_t *>(dst), src_scales, dst_scales, expert_ids,
         expert_pos, offsets, recv_counts, perm_row, world, capacity, top_k, row_bytes, cols,
-        src_scale_stride > 0 ? src_scale_stride : cols, offset_stride, static_cast<std::uint32_t *>(dst_packed), status);
+        src_scale_stride > 0 ? src_scale_stride : cols, offset_stride, static_cast<std::uint32_t *>(dst_packed),
+        status);
     return ab::launch_result("permute");
 }
 
@@ -1859,20 +1864,22 @@ AB_EXPORT int ab_permute(const void *src, void *dst, const float *src_scales, fl
                          const unsigned long long *recv_counts, int *perm_row, int world,
                          int capacity, int top_k, int row_bytes, int cols, int src_scale_stride,
                          int offset_stride, cudaStream_t stream) {
-    return launch_permute(src, dst, src_scales, dst_scales, expert_ids, expert_pos, offsets, recv_counts, perm_row, world,
-                          capacity, top_k, row_bytes, cols, src_scale_stride, offset_stride, nullptr, nullptr, stream);
+    return launch_permute(src, dst, src_scales, dst_scales, expert_ids, expert_pos, offsets, recv_counts, perm_row,
+                          world, capacity, top_k, row_bytes, cols, src_scale_stride, offset_stride, nullptr, nullptr,
+                          stream);
 }
 
 // The same with the scales packed for a block-scaled product (cols = row bytes / 128 scales per row).
 AB_EXPORT int ab_permute_packed(const void *src, void *dst, const float *src_scales, void *dst_packed,
                                 const int *expert_ids, const int *expert_pos, const int *offsets,
-                                const unsigned long long *recv_counts, int world, int capacity, int top_k, int row_bytes,
-                                int cols, int src_scale_stride, int offset_stride, unsigned long long *status,
-                                cudaStream_t stream) {
+                                const unsigned long long *recv_counts, int world, int capacity, int top_k,
+                                int row_bytes, int cols, int src_scale_stride, int offset_stride,
+                                unsigned long long *status, cudaStream_t stream) {
     if (src_scales == nullptr || dst_packed == nullptr || cols != row_bytes / 128 || row_bytes % 128)
         return -1;
-    return launch_permute(src, dst, src_scales, nullptr, expert_ids, expert_pos, offsets, recv_counts, nullptr, world,
-                          capacity, top_k, row_bytes, cols, src_scale_stride, offset_stride, dst_packed, status, stream);
+    return launch_permute(src, dst, src_scales, nullptr, expert_ids, expert_pos, offsets, recv_counts, nullptr,
+                          world, capacity, top_k, row_bytes, cols, src_scale_stride, offset_stride, dst_packed, status,
+                          stream);
 }
 
 AB_EXPORT int ab_unpermute(const void *y, void *out, const int *expert_ids, const int *expert_pos,

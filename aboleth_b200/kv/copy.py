@@ -12,8 +12,7 @@ from ..ops._kernels import _I, _U64, _VP, call, call_rc, declare, ptr, stream_pt
 declare("ab_kv_push", [_VP, _VP, _VP, _VP, _I, _U64, _I, _I, _VP, _VP])
 declare("ab_kv_push_observed", [_VP, _VP, _VP, _VP, _I, _U64, _I, _I, _VP, _VP, _U64, _VP, _VP])
 declare("ab_kv_wait", [_VP, _I, _U64, _U64, _VP, _VP])
-declare("ab_kv_push_pages", [_VP, _VP, _I, _VP, _I, _I, _U64, _U64, _U64, _U64, _U64, _U64, _I, _U64, _VP, _VP, _I, _I, _VP,
-                             _VP])
+declare("ab_kv_push_pages", [_VP, _VP, _I, _VP, _I, _I] + [_U64] * 6 + [_I, _U64, _VP, _VP, _I, _I, _VP, _VP])
 declare("ab_memcpy_async", [_VP, _VP, _U64, _VP])
 
 

@@ -36,8 +36,8 @@ def router_topk(logits: torch.Tensor, top_k: int, *, renormalize: bool = False
     tokens, experts = logits.shape
     ids = torch.empty(tokens, top_k, dtype=torch.int32, device=logits.device)
     weights = torch.empty(tokens, top_k, dtype=torch.float32, device=logits.device)
-    call("ab_router_topk" if logits.dtype == torch.float32 else "ab_router_topk_bf16", ptr(logits), ptr(ids), ptr(weights), tokens, experts, top_k,
-         int(renormalize), stream_ptr())
+    entry = "ab_router_topk" if logits.dtype == torch.float32 else "ab_router_topk_bf16"
+    call(entry, ptr(logits), ptr(ids), ptr(weights), tokens, experts, top_k, int(renormalize), stream_ptr())
     return ids, weights
 
 
