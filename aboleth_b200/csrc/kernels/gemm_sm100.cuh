@@ -61,7 +61,7 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // A whole warp waits and takes one way out, also where the wait runs out, or sees `abort`, for some lanes only.
-__device__ __forceinline__ bool warp_wait(std::uint64_t *bar, unsigned parity, const volatile int *abort) {
+__device__ __forceinline__ bool warp_wait(std::uint64_t *bar, unsigned parity, const volatile int *abort = nullptr) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort));
 }
 
