@@ -699,9 +699,14 @@ AB_EXPORT int ab_gemm_e4m3(const void *a, const void *b, void *c, int m, int n, 
 namespace {
 
 // 256-row pair tiles or 128-row tiles of single CTAs.  A pair takes 512 cycles per K step of its tile, a CTA 768
-// (it loads 48 KiB, at 64 bytes a cycle), so two CTAs are ahead where one 128-row tile holds an expert's rows
-// and behind from two on; ragged ends put the line between.
-bool pair_tiles(int total_rows, int experts) { return total_rows / experts >= 192; }
+// (it loads 48 KiB, at 64 bytes a cycle), so two CTAs are ahead where one 128-row tile holds an expert's rows and the pair
+// where it takes two of them; ragged ends put the line between.  Three 128-row tiles beat two pairs' (257 to 384 rows):
+// 8 experts x 320 rows x 4096 x 4096 bf16 102 us against 109, with SwiGLU 113 and 131, block-scaled 69 and 76; 450 rows
+// 142 against 126, 148 and 128, 84 and 79.
+bool pair_tiles(int total_rows, int experts) {
+    const int rows = total_rows / experts;
+    return rows >= 192 && (rows <= 256 || rows > 384);
+}
 
 bool grouped_ok(const void *a, const void *w, const void *c, int experts, int total_rows, int n, int k) {
     return experts >= 1 && total_rows >= 1 && n >= 1 && k >= 1 && k % 8 == 0 && n % 8 == 0 &&
@@ -710,6 +715,11 @@ bool grouped_ok(const void *a, const void *w, const void *c, int experts, int to
 }
 
 }  // namespace
+
+// Whether the grouped products of this size run on CTA pairs.
+AB_EXPORT int ab_grouped_pairs(int total_rows, int experts) {
+    return total_rows < 1 || experts < 1 ? -1 : pair_tiles(total_rows, experts);
+}
 
 // Grouped GEMM over `experts` problems that share N and K.  a: [total_rows, K],
 // w: [experts, N, K], c: [total_rows, N]; counts/offsets: device int32 [experts].

@@ -14,6 +14,7 @@ declare("ab_grouped_gemm_bf16", [_VP] * 5 + [_I] * 4 + [_VP, _VP])
 declare("ab_grouped_gemm_swiglu_bf16", [_VP] * 5 + [_I] * 4 + [_VP, _VP])
 declare("ab_gemm_split", [_I] + [_VP] * 5 + [_I] * 6 + [ctypes.c_float] + [_I] * 2 + [_VP, _VP])
 declare("ab_gemm_choice", [_I] * 4 + [_VP])
+declare("ab_grouped_pairs", [_I] * 2)
 declare("ab_gemm_e4m3", [_VP, _VP, _VP] + [_I] * 6 + [ctypes.c_float, _VP, _VP])
 
 _status: dict[torch.device, torch.Tensor] = {}

@@ -123,3 +123,12 @@ def test_packed_scale_sizes_are_those_of_the_library():
                 for which in (0, 1):
                     assert _mx_scale_bytes(m, n, k, which) == native(m, n, k, which), (m, n, k, which)
                 assert mx_scale_bytes(m, k) == native(m, n, k, 0)
+
+
+def test_grouped_products_take_pairs_where_they_win():
+    """Rows per expert on both sides of every line of the rule."""
+    from aboleth_b200.ops._kernels import call_rc
+
+    for experts in (1, 8, 64):
+        for rows, pairs in ((1, 0), (128, 0), (191, 0), (192, 1), (256, 1), (257, 0), (384, 0), (385, 1), (4096, 1)):
+            assert call_rc("ab_grouped_pairs", rows * experts, experts) == pairs

@@ -249,6 +249,7 @@ def test_grouped_swiglu_gemm_matches_fp32(counts, n, k):
 
 
 @pytest.mark.parametrize("counts,n,k", [([0, 5, 128, 200, 1, 131], 384, 384), ([700, 0, 300], 128, 128),
+                                        ([700, 0, 500], 128, 128),              # pairs, as the next
                                         ([1000, 1281, 897, 640], 2048, 128)])   # 256 pair tiles on 74 pairs
 def test_grouped_swiglu_block_scaled_gemm_is_its_parts(counts, n, k):
     """The fused gate / up product and its quantisation against the separate passes: block-scaled product, SiLU and
@@ -452,19 +453,20 @@ def test_dense_gemm_agrees_across_its_dispatch(kind, m):
     assert torch.equal(wide[:, :n], (a @ b.t()).to(torch.bfloat16)) and bool((wide[:, n:] == 7.0).all())
 
 
-@pytest.mark.parametrize("counts", [[129, 0, 1, 770], [256, 512, 255, 257]])
+@pytest.mark.parametrize("counts", [[129, 0, 1, 1153], [256, 512, 255, 513], [129, 0, 1, 770], [256, 512, 255, 257]])
 @pytest.mark.parametrize("n", [128, 640])
 def test_grouped_pair_tiles_at_their_edges(counts, n):
     """Experts just over and under a 256-row pair tile, one with a single row, one column tile that is half full:
     small integers are exact in both operand types.  (At most one tile per pair here.)"""
     from aboleth_b200.ops import check_gemm_status, grouped_gemm_bf16, grouped_gemm_e4m3_mx, pack_scales_mx
+    from aboleth_b200.ops._kernels import call_rc
 
     experts, k = len(counts), 256
     counts = torch.tensor(counts, dtype=torch.int32, device="cuda")
     padded = (counts + 127) // 128 * 128
     offsets = (torch.cumsum(padded, 0) - padded).to(torch.int32)
     rows = int(padded.sum())
-    assert rows // experts >= 192  # the pair loops
+    assert call_rc("ab_grouped_pairs", rows, experts) == (rows // experts > 384)   # the last two: the one-CTA loops
     g = torch.Generator(device="cuda").manual_seed(37)
     a = torch.randint(-2, 3, (rows, k), generator=g, device="cuda").float()
     w = torch.randint(-2, 3, (experts, n, k), generator=g, device="cuda").float()
